@@ -53,13 +53,21 @@ struct GroupSet {
   int4 *d_mem = nullptr;
   float2 *d_grppos = nullptr;
   int *d_memgrp = nullptr;
+  // queue counter, deferred-tile count, finished parts of every tile
   int *d_tile_ctr = nullptr;
+  size_t ctr_cap = 0;
+  int *d_ndefer = nullptr;  // d_tile_ctr + 1
   int *d_defer = nullptr;
   size_t defer_cap = 0;
-  int *d_ndefer = nullptr;
+  float *d_part = nullptr;  // sums of a split image's member parts
+  size_t part_cap = 0;
   int *d_nmem = nullptr;
   void *d_cub = nullptr;
 };
+// Most parts a tile's members are split into, members of a part's chunks at
+// most, and the most sums that the parts of an image leave (32 MB per set).
+constexpr int kMaxSplit = 32, kSplitChunk = 256;
+constexpr size_t kSplitSums = 1 << 23;
 
 struct PhysicsState {
   int nfft = 0, nffti = 0, nbins = 0, max_batch = 0, dtype = 0;
@@ -76,10 +84,12 @@ struct PhysicsState {
     qpsdm_ttt_desc *dt = nullptr, *dq = nullptr;
     float *ttt = nullptr, *qqq = nullptr;
     size_t dt_cap = 0, dq_cap = 0, ttt_cap = 0, qqq_cap = 0;
-    // batched form, t and t* tables with identical descriptors: (t, t*) pairs
-    float2 *tq = nullptr;
+    // batched form, t and t* tables with identical descriptors: (t, t*) of a
+    // node and of the node below it
+    float4 *tq = nullptr;
     size_t tq_cap = 0;
     bool paired = false;
+    bool one_grid = false;  // every cell has the same surface grid
   };
   std::vector<LineTab> tabs;  // one per line of the brick
   float *d_tab_tmp = nullptr;  // batched form: table upload before the re-layout
@@ -101,6 +111,8 @@ struct PhysicsState {
   int *d_defer = nullptr;    // tiles the fast form leaves to k_image_batched
   size_t defer_cap = 0;
   int *d_ndefer = nullptr;
+  float *d_part = nullptr;
+  size_t part_cap = 0;
   int *d_nmem = nullptr;                       // accepted members of the current line's batch
   void *d_cub = nullptr;
   size_t cub_bytes = 0;
@@ -139,6 +151,8 @@ static void select_set(PhysicsState *s, int i) {
   s->d_defer = g.d_defer;
   s->defer_cap = g.defer_cap;
   s->d_ndefer = g.d_ndefer;
+  s->d_part = g.d_part;
+  s->part_cap = g.part_cap;
   s->d_nmem = g.d_nmem;
   s->d_cub = g.d_cub;
   s->cur_set = i;
@@ -263,7 +277,7 @@ void physics_destroy(PhysicsState *s) {
     cudaFree(g.d_memgrp);
     cudaFree(g.d_tile_ctr);
     cudaFree(g.d_defer);
-    cudaFree(g.d_ndefer);
+    cudaFree(g.d_part);
     cudaFree(g.d_nmem);
     cudaFree(g.d_cub);
   }
@@ -332,14 +346,6 @@ static int check_tables(const qpsdm_line_params &l, std::string *err) {
 // fastest), so that image points of neighbouring cdps, which a warp of the
 // batched kernel holds, read neighbouring table words.  Out of place:
 // descriptors may share a block.
-// (t, t*) pairs of two tables with identical descriptors.
-__global__ void k_tab_pair(const float *__restrict__ t, const float *__restrict__ q,
-                           float2 *__restrict__ tq, int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    tq[i] = make_float2(t[i], q[i]);
-}
-
 __global__ void k_tab_xfast(const float *__restrict__ in, float *__restrict__ out,
                             const qpsdm_ttt_desc *__restrict__ desc, int nxi1, int nzi1) {
   const qpsdm_ttt_desc d = desc[blockIdx.y];
@@ -353,8 +359,50 @@ __global__ void k_tab_xfast(const float *__restrict__ in, float *__restrict__ ou
   }
 }
 
-// Table data may be host or device memory (cudaMemcpyDefault: unified
-// addressing tells them apart); descriptors are host memory.
+// Two tables with identical descriptors as one array of (t, t*) of a node and
+// (t, t*) of the node below it, in the cdp-fastest layout: a receiver's lookup
+// at both depth nodes of a point is four 16-byte loads instead of eight 8-byte
+// ones.  Below a cell's last node comes the first node of the cell under it
+// (on the same surface grid; else, and below the deepest cell, the node
+// itself, whose weight is zero).
+__global__ void k_tab_quads(const float *__restrict__ t, const float *__restrict__ q,
+                            float4 *__restrict__ out, const qpsdm_ttt_desc *__restrict__ desc,
+                            int nzg, int nxi1, int nzi1) {
+  const int c = blockIdx.y;
+  const qpsdm_ttt_desc d = desc[c];
+  const int nplanes = (int)d.nys * d.nxs, plane = nxi1 * nzi1;
+  int64_t under = -1;
+  if ((c + 1) % nzg != 0) {
+    const qpsdm_ttt_desc e = desc[c + 1];
+    if (e.nys == d.nys && e.nxs == d.nxs && e.dys == d.dys && e.dxs == d.dxs) under = e.idx;
+  }
+  for (int pl = blockIdx.x; pl < nplanes; pl += gridDim.x) {
+    const int64_t base = d.idx + (int64_t)pl * plane, ub = under + (int64_t)pl * plane;
+    for (int o = threadIdx.x; o < plane; o += blockDim.x) {
+      const int izl = o / nxi1, ixl = o - izl * nxi1;
+      const int64_t i = base + ixl * nzi1 + izl;
+      const int64_t j = izl + 1 < nzi1 ? i + 1 : under >= 0 ? ub + ixl * nzi1 : i;
+      out[base + o] = make_float4(t[i], q[i], t[j], q[j]);
+    }
+  }
+}
+
+// Whether no two cells of a line's traveltime tables share data: with more than
+// one depth cell, a shared block may have different cells under it.
+static bool disjoint_blocks(const qpsdm_line_params &l) {
+  std::vector<std::pair<int64_t, int64_t>> b((size_t)l.nxg * l.nzg);
+  for (size_t c = 0; c < b.size(); ++c) {
+    const qpsdm_ttt_desc &d = l.ttt_desc[c];
+    b[c] = {d.idx, d.idx + (int64_t)d.nys * d.nxs * l.nxi1 * l.nzi1};
+  }
+  std::sort(b.begin(), b.end());
+  for (size_t c = 1; c < b.size(); ++c)
+    if (b[c].first < b[c - 1].second) return false;
+  return true;
+}
+
+// Table data may be host memory or memory of the engine's device; descriptors
+// are host memory.
 int physics_set_lines(PhysicsState *s, const qpsdm_static_params &p,
                       const qpsdm_line_params *lines, int nlines, cudaStream_t st,
                       std::string *err) {
@@ -364,39 +412,70 @@ int physics_set_lines(PhysicsState *s, const qpsdm_static_params &p,
     if (rc) return rc;
   }
   if ((int)s->tabs.size() < nlines) s->tabs.resize(nlines);
+  int dev = 0;
+  cudaGetDevice(&dev);
+  // data already in this device's memory is read in place
+  auto on_device = [](const float *p, int d) -> const float * {
+    cudaPointerAttributes at;
+    const bool yes = cudaPointerGetAttributes(&at, p) == cudaSuccess &&
+                     at.type == cudaMemoryTypeDevice && at.device == d;
+    cudaGetLastError();  // a pageable pointer may leave an error behind
+    return yes ? p : nullptr;
+  };
   for (int il = 0; il < nlines; ++il) {
     const qpsdm_line_params &l = lines[il];
     PhysicsState::LineTab &t = s->tabs[il];
     const size_t ncell = (size_t)l.nxg * l.nzg;
+    t.one_grid = true;
+    for (size_t c = 0; c < ncell && t.one_grid; ++c)
+      t.one_grid = l.ttt_desc[c].nxs == l.ttt_desc[0].nxs &&
+                   l.ttt_desc[c].nys == l.ttt_desc[0].nys &&
+                   l.ttt_desc[c].dxs == l.ttt_desc[0].dxs &&
+                   l.ttt_desc[c].dys == l.ttt_desc[0].dys &&
+                   (int64_t)l.ttt_desc[c].nxs * l.ttt_desc[c].nys * l.nxi1 * l.nzi1 < (1ll << 30);
+    // identical descriptors (the reference writes both tables alike): t and t*
+    // of a node are read together
+    t.paired = s->form == QPSDM_FORM_BATCHED && l.ttt_len == l.qqq_len &&
+               std::memcmp(l.ttt_desc, l.qqq_desc, sizeof(qpsdm_ttt_desc) * ncell) == 0 &&
+               (l.nzg == 1 || disjoint_blocks(l));
+    // paired tables on one surface grid need no table of their own
+    const bool single = !(t.paired && t.one_grid);
     if (!grow_dev(&t.dt, &t.dt_cap, ncell) || !grow_dev(&t.dq, &t.dq_cap, ncell) ||
-        !grow_dev(&t.ttt, &t.ttt_cap, (size_t)l.ttt_len) ||
-        !grow_dev(&t.qqq, &t.qqq_cap, (size_t)l.qqq_len)) {
+        (single && (!grow_dev(&t.ttt, &t.ttt_cap, (size_t)l.ttt_len) ||
+                    !grow_dev(&t.qqq, &t.qqq_cap, (size_t)l.qqq_len)))) {
       if (err) *err = "table allocation failed";
       return QPSDM_ENOMEM;
     }
     cudaMemcpyAsync(t.dt, l.ttt_desc, sizeof(qpsdm_ttt_desc) * ncell, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(t.dq, l.qqq_desc, sizeof(qpsdm_ttt_desc) * ncell, cudaMemcpyHostToDevice, st);
     if (s->form == QPSDM_FORM_BATCHED) {
-      if (!grow_dev(&s->d_tab_tmp, &s->tab_tmp_cap,
-                    (size_t)std::max(l.ttt_len, l.qqq_len))) {
-        if (err) *err = "table re-layout scratch allocation failed";
-        return QPSDM_ENOMEM;
-      }
       const dim3 g(256, (unsigned)ncell);
-      cudaMemcpyAsync(s->d_tab_tmp, l.ttt, sizeof(float) * l.ttt_len, cudaMemcpyDefault, st);
-      k_tab_xfast<<<g, 256, 0, st>>>(s->d_tab_tmp, t.ttt, t.dt, l.nxi1, l.nzi1);
-      cudaMemcpyAsync(s->d_tab_tmp, l.qqq, sizeof(float) * l.qqq_len, cudaMemcpyDefault, st);
-      k_tab_xfast<<<g, 256, 0, st>>>(s->d_tab_tmp, t.qqq, t.dq, l.nxi1, l.nzi1);
-      // identical descriptors (the reference writes both tables alike): the
-      // image kernel reads t and t* of a node with one 8-byte load
-      t.paired = l.ttt_len == l.qqq_len &&
-                 std::memcmp(l.ttt_desc, l.qqq_desc, sizeof(qpsdm_ttt_desc) * ncell) == 0;
+      const float *src[2] = {on_device(l.ttt, dev), on_device(l.qqq, dev)};
+      if (!src[0] || !src[1]) {
+        if (!grow_dev(&s->d_tab_tmp, &s->tab_tmp_cap, (size_t)(l.ttt_len + l.qqq_len))) {
+          if (err) *err = "table re-layout scratch allocation failed";
+          return QPSDM_ENOMEM;
+        }
+        if (!src[0]) {
+          cudaMemcpyAsync(s->d_tab_tmp, l.ttt, sizeof(float) * l.ttt_len, cudaMemcpyDefault, st);
+          src[0] = s->d_tab_tmp;
+        }
+        if (!src[1]) {
+          cudaMemcpyAsync(s->d_tab_tmp + l.ttt_len, l.qqq, sizeof(float) * l.qqq_len,
+                          cudaMemcpyDefault, st);
+          src[1] = s->d_tab_tmp + l.ttt_len;
+        }
+      }
       if (t.paired) {
         if (!grow_dev(&t.tq, &t.tq_cap, (size_t)l.ttt_len)) {
           if (err) *err = "paired table allocation failed";
           return QPSDM_ENOMEM;
         }
-        k_tab_pair<<<148 * 8, 256, 0, st>>>(t.ttt, t.qqq, t.tq, l.ttt_len);
+        k_tab_quads<<<g, 256, 0, st>>>(src[0], src[1], t.tq, t.dt, l.nzg, l.nxi1, l.nzi1);
+      }
+      if (single) {
+        k_tab_xfast<<<g, 256, 0, st>>>(src[0], t.ttt, t.dt, l.nxi1, l.nzi1);
+        k_tab_xfast<<<g, 256, 0, st>>>(src[1], t.qqq, t.dq, l.nxi1, l.nzi1);
       }
     } else {
       cudaMemcpyAsync(t.ttt, l.ttt, sizeof(float) * l.ttt_len, cudaMemcpyDefault, st);
@@ -421,11 +500,16 @@ int physics_begin_offset(PhysicsState *s, const qpsdm_static_params &p,
   }
   if (s->form == QPSDM_FORM_BATCHED) {
     const size_t nxb = (size_t)(o.ixend - o.ixstart);
-    for (GroupSet &g : s->sets)
-      if (!grow_dev(&g.d_defer, &g.defer_cap, nxb * p.nzi / 32 + nxb + p.nzi + 1)) {
-        if (err) *err = "deferred-tile list allocation failed";
+    const size_t npt = nxb * p.nzi, ntile = npt / 32 + nxb + p.nzi + 1;  // tiles: 32 points or more
+    for (GroupSet &g : s->sets) {
+      if (!grow_dev(&g.d_defer, &g.defer_cap, ntile) ||
+          !grow_dev(&g.d_tile_ctr, &g.ctr_cap, 2 + ntile) ||
+          !grow_dev(&g.d_part, &g.part_cap, std::min(kMaxSplit * npt, kSplitSums))) {
+        if (err) *err = "tile queue allocation failed";
         return QPSDM_ENOMEM;
       }
+      g.d_ndefer = g.d_tile_ctr + 1;
+    }
     select_set(s, s->cur_set);
   }
   if (p.kahan) {
@@ -830,10 +914,11 @@ __device__ __forceinline__ bool lookup_tq(const PointCells &pc,
 
 // lookup_tq for a line whose t and t* tables have identical descriptors,
 // read as (t, t*) pairs (tq): same values, same arithmetic, half the loads.
-__device__ __forceinline__ float2 bilin2(const float2 *__restrict__ tab, int64_t base, int64_t sx,
+__device__ __forceinline__ float2 bilin2(const float4 *__restrict__ tab, int64_t base, int64_t sx,
                                          int64_t sy, float wx, float wy) {
-  const float2 v00 = __ldg(tab + base), v01 = __ldg(tab + base + sx);
-  const float2 v10 = __ldg(tab + base + sy), v11 = __ldg(tab + base + sy + sx);
+  auto ld = [&](int64_t i) { return __ldg(reinterpret_cast<const float2 *>(tab + i)); };
+  const float2 v00 = ld(base), v01 = ld(base + sx);
+  const float2 v10 = ld(base + sy), v11 = ld(base + sy + sx);
   return make_float2(lerp(lerp(v00.x, v01.x, wx), lerp(v10.x, v11.x, wx), wy),
                      lerp(lerp(v00.y, v01.y, wx), lerp(v10.y, v11.y, wx), wy));
 }
@@ -842,7 +927,7 @@ __device__ __forceinline__ bool lookup_tq(const PointCells &pc,
                                           const float *__restrict__ ttt,
                                           const qpsdm_ttt_desc *__restrict__ dq,
                                           const float *__restrict__ qqq,
-                                          const float2 *__restrict__ tq, int nxi1, int nzi1,
+                                          const float4 *__restrict__ tq, int nxi1, int nzi1,
                                           float px, float py, float &t, float &q) {
   if (!tq || !pc.same) return lookup_tq(pc, dt, ttt, dq, qqq, nxi1, nzi1, px, py, t, q);
   const int nxs = pc.nxs, nys = pc.nys;
@@ -1196,6 +1281,35 @@ __device__ __forceinline__ float block_min(float v, float (*red)[NW], int k) {
   return v;
 }
 
+// A tile whose members are split into parts: true on every thread of the CTA
+// whose part is the last one written (every part's sums are then visible).
+__device__ __forceinline__ bool last_part(int *done, int nsplit, int *s_flag) {
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) *s_flag = atomicAdd(done, 1);
+  __syncthreads();
+  if (*s_flag != nsplit - 1) return false;
+  __threadfence();
+  return true;
+}
+// Adds a point's nsplit partial sums to the image in order.
+__device__ __forceinline__ void add_parts(float *img, float *comp, const float *part, size_t nimg,
+                                          int nsplit) {
+  float s = *img, c = comp ? *comp : 0.0f;
+  for (int i = 0; i < nsplit; ++i) {
+    const float v = __ldcg(part + i * nimg);
+    if (comp) {
+      const float y = v - c, tt = s + y;
+      c = (tt - s) - y;
+      s = tt;
+    } else {
+      s += v;
+    }
+  }
+  *img = s;
+  if (comp) *comp = c;
+}
+
 // Batched imaging.  A persistent CTA takes image tiles of TZ depths x TX
 // cdps (one thread per point) from a counter.  Per tile and per chunk of sc
 // sources: the source terms of every point in shared memory; then the
@@ -1211,7 +1325,10 @@ __device__ __forceinline__ float block_min(float v, float (*red)[NW], int k) {
 // test per member decides that for the whole tile, members outside the grid
 // are dropped too, and a member dropped by the dip bound counts its
 // in-aperture points; in any other tile every member goes to the points,
-// which count for themselves.
+// which count for themselves.  nsplit > 1: an item of the queue is one of
+// nsplit parts of a tile's members (small images have fewer tiles than the
+// GPU has room for); a part leaves its sums in part[], and the part that
+// finishes a tile last adds all of them to the image in order.
 template <int TZ, int TX, int MB, int U, typename T>
 __global__ void __launch_bounds__(TZ *TX, MB)
     k_image_batched(float *__restrict__ img, float *__restrict__ comp, PhysImageArgs a,
@@ -1221,20 +1338,21 @@ __global__ void __launch_bounds__(TZ *TX, MB)
                     const float2 *__restrict__ srcpos, const int *__restrict__ nsrc_ptr,
                     const qpsdm_ttt_desc *__restrict__ dt, const float *__restrict__ ttt,
                     const qpsdm_ttt_desc *__restrict__ dq, const float *__restrict__ qqq,
-                    const float2 *__restrict__ tqp, const T *__restrict__ panels,
+                    const float4 *__restrict__ tqp, const T *__restrict__ panels,
                     int *__restrict__ tile_ctr, int ntz, int ntx, int sc,
                     unsigned long long *npt, const int *__restrict__ tile_list,
-                    const int *__restrict__ ntile_list) {
+                    const int *__restrict__ ntile_list, int nsplit, float *__restrict__ part,
+                    int *__restrict__ tile_done) {
   constexpr int NT = TZ * TX, NW = NT / 32, MC = 32 * NT;
   static_assert(NT % 32 == 0, "whole warps");
-  const int nmem = *nmem_ptr;  // the accepted members (sorted first)
+  const int nmem_all = *nmem_ptr;  // the accepted members (sorted first)
   extern __shared__ float2 smap[];  // [kMapN][sc][NT]
   __shared__ unsigned s_mask[NT];   // kept members of the chunk, one bit each
   __shared__ int s_col[TX + 1];     // active points of the tile's columns (prefix sums)
   __shared__ float s_red[13][NW];
   __shared__ TileGrid s_tg;         // the tile's shared surface grid (uniform tiles)
   __shared__ int s_tgw;             // the thread that writes it
-  __shared__ int s_tile;
+  __shared__ int s_tile, s_part;
   __shared__ unsigned long long s_cnt[3];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int lz = tid % TZ, lx = tid / TZ;
@@ -1246,14 +1364,17 @@ __global__ void __launch_bounds__(TZ *TX, MB)
     __syncthreads();
     if (tid == 0) {
       // the next tile: from the counter, or the next of a list of tiles
-      const int q = atomicAdd(tile_ctr, 1);
+      const int item = atomicAdd(tile_ctr, 1), q = item / nsplit;
+      s_part = item - q * nsplit;
       s_tile = tile_list ? (q < *ntile_list ? tile_list[q] : ntz * ntx) : q;
       s_tgw = -1;
     }
     if (tid <= TX) s_col[tid] = 0;
     __syncthreads();
-    const int tile = s_tile;
+    const int tile = s_tile, ipart = s_part;
     if (tile >= ntz * ntx) break;
+    // this item's members: chunks ipart, ipart + nsplit, ... of clen each
+    const int clen = nsplit > 1 ? min(kSplitChunk, (nmem_all + nsplit - 1) / nsplit) : MC;
     const int iz0 = (tile % ntz) * TZ, ixb0 = (tile / ntz) * TX;
     const int izi = iz0 + lz;
     const int ixb = ixb0 + lx;
@@ -1269,8 +1390,10 @@ __global__ void __launch_bounds__(TZ *TX, MB)
       tanx2 = dips[a.nxz + k];
       tany1 = dips[2 * a.nxz + k];
       tany2 = dips[3 * a.nxz + k];
-      acc = img[(size_t)ixb * a.nzi + izi];
-      if (comp) cmp = comp[(size_t)ixb * a.nzi + izi];
+      if (nsplit == 1) {
+        acc = img[(size_t)ixb * a.nzi + izi];
+        if (comp) cmp = comp[(size_t)ixb * a.nzi + izi];
+      }
       setup_cells(pc, ixi, z, a, dt, dq);
     }
     const bool act = live && pc.ok;
@@ -1361,7 +1484,8 @@ __global__ void __launch_bounds__(TZ *TX, MB)
         m[kMapPX * sc * NT] = make_float2(fmaf(-tanx1c, az, ax), fmaf(tanx2c, az, -ax));
         m[kMapPY * sc * NT] = make_float2(fmaf(-tany1c, az, ay), fmaf(tany2c, az, -ay));
       }
-      for (int pc0 = 0; pc0 < nmem; pc0 += MC) {
+      for (int pc0 = ipart * clen; pc0 < nmem_all; pc0 += nsplit * clen) {
+        const int nmem = min(pc0 + clen, nmem_all);
         // the chunk's members kept for this tile (warp w, round k: word k NW + w)
 #pragma unroll 4
         for (int k = 0; k < MC / NT; ++k) {
@@ -1534,89 +1658,150 @@ __global__ void __launch_bounds__(TZ *TX, MB)
         __syncthreads();  // the mask is rewritten by the next chunk
       }
     }
-    if (live) {
-      img[(size_t)ixb * a.nzi + izi] = acc;
-      if (comp) comp[(size_t)ixb * a.nzi + izi] = cmp;
+    const size_t o = (size_t)ixb * a.nzi + izi;
+    if (nsplit == 1) {
+      if (live) {
+        img[o] = acc;
+        if (comp) comp[o] = cmp;
+      }
+      continue;
     }
+    const size_t nimg = (size_t)a.nxb * a.nzi;
+    if (live) part[ipart * nimg + o] = acc - cmp;
+    if (!last_part(tile_done + tile, nsplit, &s_tile)) continue;
+    if (live) add_parts(img + o, comp ? comp + o : nullptr, part + o, nimg, nsplit);
   }
   if (npt) add_counts(npt, s_cnt, cnt + cdrop, cdrop, cimg);
 }
 
-// Receiver (or source) lookup of a point in a uniform tile with paired
-// (t, t*) tables: the tile's surface grid g, the point's two depth-node
-// blocks pA, pB (the cell's data plus the point's offset inside a surface
-// node's plane) and its depth weight c2.  The arithmetic of lookup_tq.
-__device__ __forceinline__ bool lookup_uni(const TileGrid &g, const float2 *__restrict__ pA,
-                                           const float2 *__restrict__ pB, float c2, int plane,
-                                           float px, float py, float &t, float &q) {
+// Surface weights of a position in a uniform tile's grid: the node offset (in
+// table pairs) and the two bilinear weights.  The arithmetic of lookup_tq; the
+// position lies on the grid (tile_covers).
+__device__ __forceinline__ void surface_weights(const TileGrid &g, float px, float py, int plane,
+                                                int &off, float &wx, float &wy) {
   float fx, fy;
-  if (!grid_pos(px, py, g.xc, g.rdx, g.rdy, g.hx, g.hy, g.nxs, g.nys, fx, fy)) return false;
+  grid_pos(px, py, g.xc, g.rdx, g.rdy, g.hx, g.hy, g.nxs, g.nys, fx, fy);
   const int ix = min((int)fx, max(g.nxs - 2, 0));
   const int iy = min((int)fy, max(g.nys - 2, 0));
-  const float wx = g.nxs > 1 ? __fsub_rn(fx, (float)ix) : 0.0f;
-  const float wy = g.nys > 1 ? __fsub_rn(fy, (float)iy) : 0.0f;
-  const int64_t sx = g.nxs > 1 ? plane : 0, sy = g.nys > 1 ? (int64_t)g.nxs * plane : 0;
-  const int64_t off = (int64_t)(iy * g.nxs + ix) * plane;
-  const float2 a = bilin2(pA, off, sx, sy, wx, wy);
-  const float2 b = bilin2(pB, off, sx, sy, wx, wy);
-  t = lerp(a.x, b.x, c2);
-  q = lerp(a.y, b.y, c2);
-  return true;
+  wx = g.nxs > 1 ? __fsub_rn(fx, (float)ix) : 0.0f;
+  wy = g.nys > 1 ? __fsub_rn(fy, (float)iy) : 0.0f;
+  off = (iy * g.nxs + ix) * plane;
+}
+
+// a + w (b - a) of a (t, t*) pair, both halves with one instruction each.
+__device__ __forceinline__ unsigned long long f2_lerp(unsigned long long a, unsigned long long b,
+                                                      unsigned long long w) {
+  return f2_fma(w, f2_sub(b, a), a);
+}
+// Bilinear (t, t*) at a point's two depth nodes (v[0] the upper) from the 2 x 2
+// surface nodes at p (bilin's arithmetic, halves packed).
+__device__ __forceinline__ void bilin_tq(const float4 *__restrict__ p, int sx, int sy,
+                                         unsigned long long wx, unsigned long long wy,
+                                         unsigned long long v[2]) {
+  const ulonglong2 *q = reinterpret_cast<const ulonglong2 *>(p);
+  const ulonglong2 v00 = __ldg(q), v01 = __ldg(q + sx);
+  const ulonglong2 v10 = __ldg(q + sy), v11 = __ldg(q + (sy + sx));
+  v[0] = f2_lerp(f2_lerp(v00.x, v01.x, wx), f2_lerp(v10.x, v11.x, wx), wy);
+  v[1] = f2_lerp(f2_lerp(v00.y, v01.y, wx), f2_lerp(v10.y, v11.y, wx), wy);
+}
+__device__ __forceinline__ unsigned long long f2_dup(float a) { return f2_pack(a, a); }
+// a + b rounded towards zero, both halves.
+__device__ __forceinline__ unsigned long long f2_add_rz(unsigned long long a,
+                                                        unsigned long long b) {
+  unsigned long long r;
+  asm("add.rz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float rsqrt_fast(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_fast(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
 
 // Batched imaging, fast form: the same sums as k_image_batched for the tiles
 // whose active points all read the same table cells of paired (t, t*)
 // tables (with the tables' x-cells and depth cells aligned to the tile shape,
 // every tile); any other tile is appended to defer[] (*ndefer of them) and
-// left to k_image_batched.  The chunk's kept members are compacted in member
-// order into shared memory (int4: trace, source slot | FP16 exponent bits,
-// tile-local column range, receiver group), so that every point reads one
-// broadcast record per member instead of scanning the keep mask and loading
-// the member from global memory; the point-traces are counted per member in
-// the keep pass (coverage is a tile-level test); lookups go through the
-// tile's surface grid in shared memory and the point's two depth-node
-// pointers.  Source terms are two float4 planes per (source, point):
-// A = (T, t* / dtstar, CS = ds^3 / ts, AZ), B = (PX1, PX2, PY1, PY2).  One
-// reciprocal per pair: inv = 1 / (uz r tt) gives both the taper's 1 / uz
-// (r tt inv) and the weight's 1 / (r tt) (uz inv), tt = t^2 (0.01 below
-// 0.1 s).  PK (two members per block): the two members' pick, weight and
-// sample blend run as packed FP32 pairs (one f32x2 instruction for both
-// members; minima, conversions and the sums stay scalar); every value that
-// decides a pair -- t, t / dt1, the t* bin -- is the same IEEE add or
-// multiply as in the scalar walk, so the same pairs are imaged.
-template <int TZ, int TX, int MB, int U, int MW, bool PK, typename T>
-__global__ void __launch_bounds__(TZ *TX, MB)
+// left to k_image_batched.
+//
+// A thread holds two neighbouring depths of one cdp, and every FP32 operation
+// of the walk runs on both in one f32x2 instruction; minima, reciprocals,
+// comparisons and panel loads stay scalar.  The kernel is bound by issued
+// instructions, and the two depths share what does not depend on depth: the
+// member record, the range test, the table nodes of the receiver (when both
+// depths lie between the same depth nodes: four pair loads and the bilinear
+// surface interpolation at two nodes serve both), the horizontal part of the
+// ray.  Integer parts (the time sample and the t* bin) come from adding 2^23
+// towards zero, which leaves floor(x) in the low mantissa bits: no conversion
+// instructions, whose unit runs at an eighth of the FP32 rate.
+//
+// The chunk's kept members are compacted in member order into shared memory:
+// a record {trace, source slot | new receiver | column bits, table offset,
+// 100 x FP16 scale} and {receiver position, surface weights}, so that every
+// point reads broadcast records and no point recomputes what is the same for
+// the tile.  Point-traces are counted per member in the keep pass (coverage
+// is a tile-level test).  Source terms are four float4 planes per (source,
+// pair of points), each holding two terms of both points: (PX1, PX2),
+// (PY1, PY2), (T, t* / dtstar), (CS = ds^3 / ts, AZ).  One reciprocal per
+// point-trace: inv = 1 / (uz r tt) gives both the taper's 1 / uz (r tt inv)
+// and the weight's 1 / (r tt) (uz inv), tt = t^2 (0.01 below 0.1 s).  Every
+// value that decides a pair -- the dip-test functions, t, t / dt1 -- is the
+// same IEEE operation as in k_image_batched.
+//
+// Measured, image kernels of a brick of four 512 x 400 lines of 18,432 traces
+// (5.8e8 kept, 4.5e8 imaged pairs a line): 21.3 ms with one point per thread
+// and two members per instruction, 11.4 ms with this walk and split parts; a
+// line alone is 3.1 ms, 229 warp instructions per member and 64 points, issue
+// active 62 %, stalls long scoreboard (table nodes, panel samples) first.
+// Loading the next receiver's nodes ahead (16 more registers, 16 warps) and
+// two members per block were slower.
+//
+// nsplit: as in k_image_batched.
+constexpr int kNewGroup = 0x100;
+template <int TZ, int TX, int MB, int U, int MW, typename T>
+__global__ void __launch_bounds__(TZ *TX / 2, MB)
     k_image_batched_fast(float *__restrict__ img, float *__restrict__ comp, PhysImageArgs a,
-                       const float *__restrict__ dips, const int *__restrict__ memgrp,
-                       const float2 *__restrict__ grppos, const int4 *__restrict__ mem,
-                       const int *__restrict__ nmem_ptr,
-                       const float2 *__restrict__ srcpos, const int *__restrict__ nsrc_ptr,
-                       const qpsdm_ttt_desc *__restrict__ dt, const float *__restrict__ ttt,
-                       const qpsdm_ttt_desc *__restrict__ dq, const float *__restrict__ qqq,
-                       const float2 *__restrict__ tqp, const T *__restrict__ panels,
-                       int *__restrict__ tile_ctr, int ntz, int ntx, int sc,
-                       unsigned long long *npt, int *__restrict__ defer,
-                       int *__restrict__ ndefer) {
-  constexpr int NT = TZ * TX, NW = NT / 32, MC = 32 * MW;
-  static_assert(NT % 32 == 0 && MW % NW == 0, "whole warps, whole words per warp");
-  const int nmem = *nmem_ptr;
-  extern __shared__ float4 smap4[];  // [2][sc][NT]: plane A, plane B
-  __shared__ int4 s_list[MC];        // the chunk's kept members, in member order
+                         const float *__restrict__ dips, const int *__restrict__ memgrp,
+                         const float2 *__restrict__ grppos, const int4 *__restrict__ mem,
+                         const int *__restrict__ nmem_ptr,
+                         const float2 *__restrict__ srcpos, const int *__restrict__ nsrc_ptr,
+                         const qpsdm_ttt_desc *__restrict__ dt,
+                         const qpsdm_ttt_desc *__restrict__ dq,
+                         const float4 *__restrict__ tqp, const T *__restrict__ panels,
+                         int *__restrict__ tile_ctr, int ntz, int ntx, int sc,
+                         unsigned long long *npt, int *__restrict__ defer,
+                         int *__restrict__ ndefer, int nsplit, float *__restrict__ part,
+                         int *__restrict__ tile_done) {
+  constexpr int NT = TZ * TX / 2, NW = NT / 32, MC = 32 * MW, HZ = TZ / 2;
+  static_assert(NT % 32 == 0 && MW % NW == 0 && TX <= 16, "whole warps, whole words per warp");
+  const int nmem_all = *nmem_ptr;
+  extern __shared__ float4 smap4[];  // [4][sc][NT]
+  __shared__ int4 s_rec[MC + U];     // the chunk's kept members, in member order
+  __shared__ float4 s_geo[MC];       // their receivers: x, y, surface weights
   __shared__ unsigned s_mask[MW];    // kept members of the chunk, one bit each
   __shared__ int s_wpos[MW + 1];     // kept members before word w (s_wpos[MW]: all)
   __shared__ int s_col[TX + 1];      // active points of the tile's columns (prefix sums)
-  __shared__ float s_red[13][NW];
+  __shared__ float s_red[14][NW];
   __shared__ TileGrid s_tg;
   __shared__ TileBox s_box;  // the tile's box and dip-limit ranges (keep pass only)
+  __shared__ int64_t s_base;
   __shared__ int s_tgw;
   __shared__ int s_tile;
   __shared__ unsigned long long s_cnt[3];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int lz = tid % TZ, lx = tid / TZ;
+  const int lz = 2 * (tid % HZ), lx = tid / HZ;
   const int nsrc = *nsrc_ptr;
   const float inv_dt1 = 1.0f / a.dt1, inv_dts = 1.0f / a.dtstar;
-  const size_t pstride = (size_t)a.nbins * a.nt;
-  float4 *const planeA = smap4, *const planeB = smap4 + (size_t)sc * NT;
+  // largest t* bin coordinate whose bin has a right neighbour
+  const float fb_max = __int_as_float(__float_as_int((float)(a.nbins - 1)) - 1);
+  const unsigned idx0 = 0x4B000000u * (unsigned)(a.nt + 1);  // 2^23's bits, of both integer parts
+  const unsigned pstride = (unsigned)a.nbins * a.nt;
+  const int splane = sc * NT;
   unsigned cnt = 0, cdrop = 0, cimg = 0;
   for (;;) {
     __syncthreads();
@@ -1626,63 +1811,97 @@ __global__ void __launch_bounds__(TZ *TX, MB)
     }
     if (tid <= TX) s_col[tid] = 0;
     __syncthreads();
-    const int tile = s_tile;
-    if (tile >= ntz * ntx) break;
+    const int item = s_tile;
+    if (item >= ntz * ntx * nsplit) break;
+    const int tile = item / nsplit, ipart = item - tile * nsplit;
+    // this item's members: chunks ipart, ipart + nsplit, ... of clen each
+    const int clen = nsplit > 1 ? min(kSplitChunk, (nmem_all + nsplit - 1) / nsplit) : MC;
     const int iz0 = (tile % ntz) * TZ, ixb0 = (tile / ntz) * TX;
     const int izi = iz0 + lz;
     const int ixb = ixb0 + lx;
-    const bool live = izi < a.nzi && ixb < a.nxb;
     const int ixi = ixb + a.ixstart;
-    PointCells pc;
-    pc.ok = false;
-    float tanx1 = 0.f, tanx2 = 0.f, tany1 = 0.f, tany2 = 0.f, acc = 0.f, cmp = 0.f;
-    const float z = izi * a.dzi;
-    if (live) {
-      const size_t k = (size_t)ixi * a.nzi + izi;
-      tanx1 = dips[k];
-      tanx2 = dips[a.nxz + k];
-      tany1 = dips[2 * a.nxz + k];
-      tany2 = dips[3 * a.nxz + k];
-      acc = img[(size_t)ixb * a.nzi + izi];
-      if (comp) cmp = comp[(size_t)ixb * a.nzi + izi];
-      setup_cells(pc, ixi, z, a, dt, dq);
-    }
-    const bool act = live && pc.ok;
-    const float tz = a.taperzone;
-    const float tanx1c = tanx1 - tz * (1.0f + tanx1 * tanx1);
-    const float tanx2c = tanx2 + tz * (1.0f + tanx2 * tanx2);
-    const float tany1c = tany1 - tz * (1.0f + tany1 * tany1);
-    const float tany2c = tany2 + tz * (1.0f + tany2 * tany2);
-    const float iwx1 = 1.0f / (tanx1 - tanx1c), iwx2 = 1.0f / (tanx2c - tanx2);
-    const float iwy1 = 1.0f / (tany1 - tany1c), iwy2 = 1.0f / (tany2c - tany2);
-    const float z2 = z * z;
     const float x = ixi * a.dxi;
+    bool live[2], act[2];
+    int off0, off1;
+    float zv[2], c2v[2], lim[4][2], iwv[4][2], accv[2], cmpv[2];
     {
+      PointCells pc[2];
+      float tc[4][2];
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        live[p] = izi + p < a.nzi && ixb < a.nxb;
+        pc[p].ok = false;
+        zv[p] = (izi + p) * a.dzi;
+        accv[p] = cmpv[p] = 0.0f;
+        float tan[4] = {0.f, 0.f, 0.f, 0.f};
+        if (live[p]) {
+          const size_t k = (size_t)ixi * a.nzi + izi + p;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) tan[j] = dips[j * a.nxz + k];
+          if (nsplit == 1) {
+            accv[p] = img[(size_t)ixb * a.nzi + izi + p];
+            if (comp) cmpv[p] = comp[(size_t)ixb * a.nzi + izi + p];
+          }
+          setup_cells(pc[p], ixi, zv[p], a, dt, dq);
+        }
+        act[p] = live[p] && pc[p].ok;
+        const float tz = a.taperzone;
+        tc[0][p] = tan[0] - tz * (1.0f + tan[0] * tan[0]);
+        tc[1][p] = tan[1] + tz * (1.0f + tan[1] * tan[1]);
+        tc[2][p] = tan[2] - tz * (1.0f + tan[2] * tan[2]);
+        tc[3][p] = tan[3] + tz * (1.0f + tan[3] * tan[3]);
+        // inverse taper-zone widths: the taper factor at a passing pair is
+        // min(1, f / (w uz)) for the test function f of each limit, w = |tan - tanc|
+        iwv[0][p] = 1.0f / (tan[0] - tc[0][p]), iwv[1][p] = 1.0f / (tc[1][p] - tan[1]);
+        iwv[2][p] = 1.0f / (tan[2] - tc[2][p]), iwv[3][p] = 1.0f / (tc[3][p] - tan[3]);
+        // a point without table values fails every dip test
+#pragma unroll
+        for (int j = 0; j < 4; ++j) lim[j][p] = act[p] ? tc[j][p] : NAN;
+      }
+      if (act[0] && !act[1]) pc[1] = pc[0];
+      off0 = pc[0].offA, off1 = pc[1].offA;
+      c2v[0] = pc[0].c2, c2v[1] = pc[1].c2;
       const float big = 3.0e38f;
-      block_min<NW>(act ? tanx1c : big, s_red, 0);
-      block_min<NW>(act ? -tanx1c : big, s_red, 1);
-      block_min<NW>(act ? tanx2c : big, s_red, 2);
-      block_min<NW>(act ? -tanx2c : big, s_red, 3);
-      block_min<NW>(act ? tany1c : big, s_red, 4);
-      block_min<NW>(act ? -tany1c : big, s_red, 5);
-      block_min<NW>(act ? tany2c : big, s_red, 6);
-      block_min<NW>(act ? -tany2c : big, s_red, 7);
-      block_min<NW>(act ? (float)pc.cA : big, s_red, 8);
-      block_min<NW>(act ? -(float)pc.cA : big, s_red, 9);
-      block_min<NW>(act ? (float)pc.cB : big, s_red, 10);
-      block_min<NW>(act ? -(float)pc.cB : big, s_red, 11);
-      block_min<NW>(act ? (pc.same ? 0.0f : -1.0f) : big, s_red, 12);
-      if (act) atomicAdd(&s_col[lx + 1], 1);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        block_min<NW>(fminf(act[0] ? tc[j][0] : big, act[1] ? tc[j][1] : big), s_red, 2 * j);
+        block_min<NW>(fminf(act[0] ? -tc[j][0] : big, act[1] ? -tc[j][1] : big), s_red, 2 * j + 1);
+      }
+      // the table cells of the tile's points (exact in float: cells < 2^24)
+      float cAl = big, cAh = big, cBl = big, cBh = big, same = big, apart = big;
+#pragma unroll
+      for (int p = 0; p < 2; ++p)
+        if (act[p]) {
+          cAl = fminf(cAl, (float)pc[p].cA), cAh = fminf(cAh, -(float)pc[p].cA);
+          cBl = fminf(cBl, (float)pc[p].cB), cBh = fminf(cBh, -(float)pc[p].cB);
+          const bool wide = (int64_t)pc[p].nxs * pc[p].nys * a.nxi1 * a.nzi1 >= (1ll << 30);
+          same = fminf(same, pc[p].same && !wide ? 0.0f : -1.0f);
+        }
+      if (act[0]) apart = off0 == off1 ? 0.0f : -1.0f;
+      block_min<NW>(cAl, s_red, 8);
+      block_min<NW>(cAh, s_red, 9);
+      block_min<NW>(cBl, s_red, 10);
+      block_min<NW>(cBh, s_red, 11);
+      block_min<NW>(same, s_red, 12);
+      block_min<NW>(apart, s_red, 13);
+      if (act[0]) {
+        atomicAdd(&s_col[lx + 1], act[1] ? 2 : 1);
+        if (atomicCAS(&s_tgw, -1, tid) == -1) {
+          s_tg = TileGrid{pc[0].xc, pc[0].rdx, pc[0].rdy, pc[0].hx, pc[0].hy, pc[0].nxs,
+                          pc[0].nys};
+          s_base = pc[0].tA;
+        }
+      }
     }
     __syncthreads();
     if (tid == 0)
       for (int c = 1; c <= TX; ++c) s_col[c] += s_col[c - 1];
-    bool uni;
+    bool uni, shared_nodes;
     {
       TileBox box;
-      float r[13];
+      float r[14];
 #pragma unroll
-      for (int k = 0; k < 13; ++k) {
+      for (int k = 0; k < 14; ++k) {
         r[k] = s_red[k][0];
 #pragma unroll
         for (int w = 1; w < NW; ++w) r[k] = fminf(r[k], s_red[k][w]);
@@ -1699,46 +1918,81 @@ __global__ void __launch_bounds__(TZ *TX, MB)
       box.z0 = iz0 * a.dzi;
       box.z1 = (iz0 + nrow - 1) * a.dzi;
       uni = r[8] == -r[9] && r[10] == -r[11] && r[12] == 0.0f;
+      shared_nodes = r[13] == 0.0f;
       if (tid == 0) s_box = box;
-      if (uni && act && atomicCAS(&s_tgw, -1, tid) == -1)
-        s_tg = TileGrid{pc.xc, pc.rdx, pc.rdy, pc.hx, pc.hy, pc.nxs, pc.nys};
     }
     __syncthreads();
     if (s_col[TX] == 0) continue;
     if (!uni) {  // left to k_image_batched
-      if (tid == 0) defer[atomicAdd(ndefer, 1)] = tile;
+      if (tid == 0 && ipart == 0) defer[atomicAdd(ndefer, 1)] = tile;
       continue;
     }
     const int ixi_lo = ixb0 + a.ixstart, ixi_hi = ixi_lo + min(TX, a.nxb - ixb0) - 1;
     const int plane = a.nxi1 * a.nzi1;
-    const float2 *ptA = tqp, *ptB = tqp;
-    if (act) {
-      ptA = tqp + pc.tA + pc.offA;
-      ptB = tqp + pc.tB + pc.offB;
-    }
-    const float c2 = pc.c2;
+    const int tsx = s_tg.nxs > 1 ? plane : 0, tsy = s_tg.nys > 1 ? s_tg.nxs * plane : 0;
+    const float4 *const tab0 = tqp + s_base + off0, *const tab1 = tqp + s_base + off1;
+    // (t, t*) of both points for a surface position
+    auto lookup = [&](int off, float wx, float wy, unsigned long long &t, unsigned long long &q) {
+      const unsigned long long wx2 = f2_dup(wx), wy2 = f2_dup(wy);
+      unsigned long long v0[2], v1[2];
+      bilin_tq(tab0 + off, tsx, tsy, wx2, wy2, v0);
+      v1[0] = v0[0], v1[1] = v0[1];
+      if (!shared_nodes) bilin_tq(tab1 + off, tsx, tsy, wx2, wy2, v1);
+      const float2 A0 = f2_unpack(v0[0]), B0 = f2_unpack(v0[1]);
+      const float2 A1 = f2_unpack(v1[0]), B1 = f2_unpack(v1[1]);
+      t = f2_pack(lerp(A0.x, B0.x, c2v[0]), lerp(A1.x, B1.x, c2v[1]));
+      q = f2_pack(lerp(A0.y, B0.y, c2v[0]), lerp(A1.y, B1.y, c2v[1]));
+    };
+    const unsigned long long zp = f2_pack(zv[0], zv[1]);
+    const unsigned long long z2p = f2_mul(zp, zp);
+    const unsigned long long nl0 = f2_pack(-lim[0][0], -lim[0][1]);
+    const unsigned long long nl1 = f2_pack(-lim[1][0], -lim[1][1]);
+    const unsigned long long nl2 = f2_pack(-lim[2][0], -lim[2][1]);
+    const unsigned long long nl3 = f2_pack(-lim[3][0], -lim[3][1]);
+    const unsigned long long iw0 = f2_pack(iwv[0][0], iwv[0][1]);
+    const unsigned long long iw1 = f2_pack(iwv[1][0], iwv[1][1]);
+    const unsigned long long iw2 = f2_pack(iwv[2][0], iwv[2][1]);
+    const unsigned long long iw3 = f2_pack(iwv[3][0], iwv[3][1]);
+    const unsigned long long two23 = f2_dup(8388608.0f);
+    unsigned long long acc = f2_pack(accv[0], accv[1]), cmp = f2_pack(cmpv[0], cmpv[1]);
+    const unsigned mybit = 0x10000u << lx;
 
     for (int s0 = 0; s0 < nsrc; s0 += sc) {
       const int ns = min(sc, nsrc - s0);
-      for (int s = 0; s < ns && act; ++s) {
+      for (int s = 0; s < ns && act[0]; ++s) {
         const float2 sp = srcpos[s0 + s];
-        float ts, qs;
-        float4 *mA = planeA + (size_t)s * NT + tid, *mB = planeB + (size_t)s * NT + tid;
-        if (!lookup_uni(s_tg, ptA, ptB, c2, plane, sp.x, sp.y, ts, qs)) {
+        float4 *m = smap4 + s * NT + tid;
+        if (!tile_covers(s_tg, sp)) {
           // no table value: NaN fails every member's dip test
-          *mA = make_float4(NAN, 0.0f, 0.0f, NAN);
-          *mB = make_float4(NAN, NAN, NAN, NAN);
+          m[0] = m[splane] = m[2 * splane] = m[3 * splane] = make_float4(NAN, NAN, NAN, NAN);
           continue;
         }
+        int off;
+        float wx, wy;
+        surface_weights(s_tg, sp.x, sp.y, plane, off, wx, wy);
+        unsigned long long tp, qp;
+        lookup(off, wx, wy, tp, qp);
+        const float2 ts = f2_unpack(tp), qs = f2_unpack(qp);
         const float dsx = sp.x - x;
-        const float ds = sqrtf(dsx * dsx + sp.y * sp.y + z2);
-        const float rds = __fdividef(1.0f, ds);
-        const float ax = dsx * rds, ay = sp.y * rds, az = z * rds;
-        *mA = make_float4(ts, qs * inv_dts, __fdividef(ds * ds * ds, ts), az);
-        *mB = make_float4(fmaf(-tanx1c, az, ax), fmaf(tanx2c, az, -ax), fmaf(-tany1c, az, ay),
-                          fmaf(tany2c, az, -ay));
+        float px1[2], px2[2], py1[2], py2[2], cs[2], azv[2];
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+          const float z2 = zv[p] * zv[p];
+          const float ds = sqrtf(dsx * dsx + sp.y * sp.y + z2);
+          const float rds = __fdividef(1.0f, ds);
+          const float ax = dsx * rds, ay = sp.y * rds, az = zv[p] * rds;
+          cs[p] = __fdividef(ds * ds * ds, p ? ts.y : ts.x);
+          azv[p] = az;
+          px1[p] = fmaf(-lim[0][p], az, ax), px2[p] = fmaf(lim[1][p], az, -ax);
+          py1[p] = fmaf(-lim[2][p], az, ay), py2[p] = fmaf(lim[3][p], az, -ay);
+        }
+        m[0] = make_float4(px1[0], px1[1], px2[0], px2[1]);
+        m[splane] = make_float4(py1[0], py1[1], py2[0], py2[1]);
+        m[2 * splane] = make_float4(ts.x, ts.y, qs.x * inv_dts, qs.y * inv_dts);
+        m[3 * splane] = make_float4(cs[0], cs[1], azv[0], azv[1]);
       }
-      for (int pc0 = 0; pc0 < nmem; pc0 += MC) {
+      for (int pc0 = ipart * clen; pc0 < nmem_all; pc0 += nsplit * clen) {
+        const int nmem = min(pc0 + clen, nmem_all);
         // keep pass: one bit per member of the chunk
 #pragma unroll 4
         for (int k = 0; k < MW / NW; ++k) {
@@ -1781,229 +2035,205 @@ __global__ void __launch_bounds__(TZ *TX, MB)
         }
         __syncthreads();
         // the kept members' records, in member order
-#pragma unroll 4
+#pragma unroll 2
         for (int k = 0; k < MW / NW; ++k) {
           const int wi = k * NW + warp;
           const unsigned bits = s_mask[wi];
           if (!((bits >> lane) & 1u)) continue;
           const int p = pc0 + 32 * wi + lane;
           const int4 mi = __ldg(mem + p);
-          const int sl = (mi.y & 0xFFFFFF) - s0;
+          const int sl = (mi.y & 0xFFFFFF) - s0, g = __ldg(memgrp + p);
+          const unsigned below = bits & ((1u << lane) - 1u);
+          // the kept member before this one, in this or an earlier word
+          int prev = -1;
+          if (below) {
+            prev = pc0 + 32 * wi + 31 - __clz(below);
+          } else {
+            for (int w = wi - 1; w >= 0; --w)
+              if (s_mask[w]) {
+                prev = pc0 + 32 * w + 31 - __clz(s_mask[w]);
+                break;
+              }
+          }
+          const bool fresh = prev < 0 || __ldg(memgrp + prev) != g;
           const int lo = max(mi.z, ixi_lo) - ixi_lo, hi = min(mi.w, ixi_hi) - ixi_lo;
-          s_list[s_wpos[wi] + __popc(bits & ((1u << lane) - 1u))] =
-              make_int4(mi.x, sl | (int)((unsigned)mi.y & 0xFF000000u), (lo << 16) | hi,
-                        __ldg(memgrp + p));
+          const unsigned cols = (0xFFFFu >> (15 - hi)) & (0xFFFFu << lo);
+          const float2 gp = __ldg(grppos + g);
+          int off;
+          float wx, wy;
+          surface_weights(s_tg, gp.x, gp.y, plane, off, wx, wy);
+          // 2^e of the trace's FP16 panel from the record's exponent bits
+          float scale = 100.0f;
+          if (std::is_same<T, __half>::value)
+            scale *= __int_as_float((int)((((unsigned)mi.y >> 24) - 1u) << 23));
+          const int at = s_wpos[wi] + __popc(below);
+          s_rec[at] = make_int4(mi.x, (int)(cols << 16) | (fresh ? kNewGroup : 0) | sl, off,
+                                __float_as_int(scale));
+          s_geo[at] = make_float4(gp.x, gp.y, wx, wy);
         }
+        if (tid < U) s_rec[s_wpos[MW] + tid] = make_int4(0, kNewGroup, 0, 0);  // ends a block
         __syncthreads();
         const int nkept = s_wpos[MW];
-        if (act && nkept > 0) {
-          int cur = -1;
-          float agz = 0.f, qx1 = 0.f, qx2 = 0.f, qy1 = 0.f, qy2 = 0.f;
-          float tg = 0.f, qg = 0.f, gfac = 0.f;
+        if (act[0] && nkept > 0) {
+          unsigned long long agz = 0, q0 = 0, q1 = 0, q2 = 0, q3 = 0, tg = 0, qg = 0, gfac = 0;
+          int4 nx = s_rec[0];
           for (int k = 0; k < nkept;) {
             int4 rec[U];
-            rec[0] = s_list[k];
-            const int g = rec[0].w;
-            if (g != cur) {
-              cur = g;
-              // receiver terms, once per receiver position (a kept member's
-              // receiver lies on the tile's surface grid)
-              const float2 gp = __ldg(grppos + g);
-              const bool rok = lookup_uni(s_tg, ptA, ptB, c2, plane, gp.x, gp.y, tg, qg);
-              const float dgx = gp.x - x;
-              const float rdg = rsqrtf(dgx * dgx + gp.y * gp.y + z2);
-              const float agx = dgx * rdg, agy = gp.y * rdg;
-              agz = z * rdg;
-              qx1 = rok ? fmaf(tanx1c, agz, -agx) : NAN;
-              qx2 = fmaf(-tanx2c, agz, agx);
-              qy1 = fmaf(tany1c, agz, -agy);
-              qy2 = fmaf(-tany2c, agz, agy);
-              gfac = tg * rdg * rdg * rdg;
-              qg *= inv_dts;
+            rec[0] = nx;
+            if (rec[0].y & kNewGroup) {
+              // receiver terms, once per receiver position
+              const float4 ge = s_geo[k];
+              lookup(rec[0].z, ge.z, ge.w, tg, qg);
+              const float dgx = ge.x - x;
+              const float2 d2 = f2_unpack(f2_add(f2_dup(dgx * dgx + ge.y * ge.y), z2p));
+              const unsigned long long rdg = f2_pack(rsqrt_fast(d2.x), rsqrt_fast(d2.y));
+              const unsigned long long agx = f2_mul(f2_dup(dgx), rdg);
+              const unsigned long long agy = f2_mul(f2_dup(ge.y), rdg);
+              agz = f2_mul(zp, rdg);
+              // dip-test thresholds of this receiver: q0, q2 with opposite sign
+              q0 = f2_fma(nl0, agz, agx);
+              q1 = f2_fma(nl1, agz, agx);
+              q2 = f2_fma(nl2, agz, agy);
+              q3 = f2_fma(nl3, agz, agy);
+              gfac = f2_mul(f2_mul(f2_mul(tg, rdg), rdg), rdg);
+              qg = f2_mul(qg, f2_dup(inv_dts));
             }
-            // up to U kept members of this receiver group
-            bool val[U];
-            val[0] = true;
+            // up to U kept members of this receiver
+            bool take[U];
+            take[0] = true;
             ++k;
+            nx = s_rec[k];
 #pragma unroll
             for (int u = 1; u < U; ++u) {
-              rec[u] = k < nkept ? s_list[k] : make_int4(0, 0, 0, -1);
-              val[u] = rec[u].w == g;
-              if (val[u]) ++k;
-            }
-            if constexpr (PK) {
-              static_assert(U == 2, "packed walk: two members per block");
-              bool on[2];
-              float4 A[2], B[2];
-#pragma unroll
-              for (int u = 0; u < 2; ++u) {
-                const int lo = rec[u].z >> 16, hi = rec[u].z & 0xFFFF;
-                const bool inr = val[u] && (unsigned)(lx - lo) <= (unsigned)(hi - lo);
-                B[u] = planeB[(size_t)(rec[u].y & 0xFF) * NT + tid];
-                on[u] = inr && B[u].x > qx1 && B[u].y > qx2 && B[u].z > qy1 && B[u].w > qy2;
+              rec[u] = nx;
+              take[u] = take[u - 1] && !(nx.y & kNewGroup);
+              if (take[u]) {
+                ++k;
+                nx = s_rec[k];
               }
-              if (!(on[0] || on[1])) continue;
+            }
+            bool on[U][2], any = false;
+            float4 F0[U], F1[U];
+            const float2 q0v = f2_unpack(q0), q1v = f2_unpack(q1);
+            const float2 q2v = f2_unpack(q2), q3v = f2_unpack(q3);
 #pragma unroll
-              for (int u = 0; u < 2; ++u) A[u] = planeA[(size_t)(rec[u].y & 0xFF) * NT + tid];
-              const unsigned long long Ax = f2_pack(A[0].x, A[1].x), Ay = f2_pack(A[0].y, A[1].y);
-              const unsigned long long Az = f2_pack(A[0].z, A[1].z), Aw = f2_pack(A[0].w, A[1].w);
-              const unsigned long long uz = f2_add(Aw, f2_pack(agz, agz));
-              const float2 ex1 = f2_unpack(f2_mul(f2_sub(f2_pack(B[0].x, B[1].x), f2_pack(qx1, qx1)),
-                                                  f2_pack(iwx1, iwx1)));
-              const float2 ex2 = f2_unpack(f2_mul(f2_sub(f2_pack(B[0].y, B[1].y), f2_pack(qx2, qx2)),
-                                                  f2_pack(iwx2, iwx2)));
-              const float2 ey1 = f2_unpack(f2_mul(f2_sub(f2_pack(B[0].z, B[1].z), f2_pack(qy1, qy1)),
-                                                  f2_pack(iwy1, iwy1)));
-              const float2 ey2 = f2_unpack(f2_mul(f2_sub(f2_pack(B[0].w, B[1].w), f2_pack(qy2, qy2)),
-                                                  f2_pack(iwy2, iwy2)));
-              const unsigned long long t = f2_add(Ax, f2_pack(tg, tg));
-              const unsigned long long ft = f2_mul(t, f2_pack(inv_dt1, inv_dt1));
-              const float2 ftv = f2_unpack(ft), tv = f2_unpack(t);
-              const float2 fbr = f2_unpack(f2_add(Ay, f2_pack(qg, qg)));
-              const int it0 = (int)ftv.x, it1v = (int)ftv.y;
-              on[0] = on[0] && it0 > 0 && it0 + 1 < a.nt;
-              on[1] = on[1] && it1v > 0 && it1v + 1 < a.nt;
-              const float fb0 = fminf(fmaxf(fbr.x, 0.0f), (float)(a.nbins - 1));
-              const float fb1 = fminf(fmaxf(fbr.y, 0.0f), (float)(a.nbins - 1));
-              const int b00 = min((int)fb0, a.nbins - 2), b01 = min((int)fb1, a.nbins - 2);
-              const unsigned long long fwt = f2_sub(ft, f2_pack((float)it0, (float)it1v));
-              const unsigned long long fwb =
-                  f2_sub(f2_pack(fb0, fb1), f2_pack((float)b00, (float)b01));
-              // w v (r + 1/r) = w (r^2 + 1) 100 / (r tt), tt = t^2 (0.01 below 0.1 s)
-              const unsigned long long r = f2_mul(Az, f2_pack(gfac, gfac));
-              const float2 t2 = f2_unpack(f2_mul(t, t));
+            for (int u = 0; u < U; ++u) {
+              const float4 *m = smap4 + (rec[u].y & 0xFF) * NT + tid;
+              F0[u] = m[0];
+              F1[u] = m[splane];
+              const bool inr = take[u] && ((unsigned)rec[u].y & mybit);
+              on[u][0] = inr && F0[u].x > -q0v.x && F0[u].z > q1v.x && F1[u].x > -q2v.x &&
+                         F1[u].z > q3v.x;
+              on[u][1] = inr && F0[u].y > -q0v.y && F0[u].w > q1v.y && F1[u].y > -q2v.y &&
+                         F1[u].w > q3v.y;
+              any = any || on[u][0] || on[u][1];
+            }
+            if (!any) continue;
+            unsigned long long fwt[U], fwb[U], fac[U];
+            const T *pp[U][2];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              const float4 *m = smap4 + (rec[u].y & 0xFF) * NT + tid;
+              const float4 F2 = m[2 * splane], F3 = m[3 * splane];
+              const unsigned long long t = f2_add(f2_pack(F2.x, F2.y), tg);
+              const unsigned long long ft = f2_mul(t, f2_dup(inv_dt1));
+              // floor in the low bits (ft < 0 and NaN fail the window test)
+              const unsigned long long mt = f2_add_rz(ft, two23);
+              fwt[u] = f2_sub(ft, f2_sub(mt, two23));
+              const float2 fbr = f2_unpack(f2_add(f2_pack(F2.z, F2.w), qg));
+              const unsigned long long fb = f2_pack(fminf(fmaxf(fbr.x, 0.0f), fb_max),
+                                                    fminf(fmaxf(fbr.y, 0.0f), fb_max));
+              const unsigned long long mb = f2_add_rz(fb, two23);
+              fwb[u] = f2_sub(fb, f2_sub(mb, two23));
+              const float2 mtv = f2_unpack(mt), mbv = f2_unpack(mb);
+              const unsigned it0 = __float_as_uint(mtv.x), it1 = __float_as_uint(mtv.y);
+              on[u][0] = on[u][0] && it0 - 0x4B000001u < (unsigned)(a.nt - 2);
+              on[u][1] = on[u][1] && it1 - 0x4B000001u < (unsigned)(a.nt - 2);
+              const T *pt = panels + (uint64_t)(unsigned)rec[u].x * pstride;
+              pp[u][0] = pt + (__float_as_uint(mbv.x) * (unsigned)a.nt + it0 - idx0);
+              pp[u][1] = pt + (__float_as_uint(mbv.y) * (unsigned)a.nt + it1 - idx0);
+              // dip taper and w v (r + 1/r) = w (r^2 + 1) 100 / (r tt)
+              const unsigned long long uz = f2_add(f2_pack(F3.z, F3.w), agz);
+              const float2 e0 = f2_unpack(f2_mul(f2_add(f2_pack(F0[u].x, F0[u].y), q0), iw0));
+              const float2 e1 = f2_unpack(f2_mul(f2_sub(f2_pack(F0[u].z, F0[u].w), q1), iw1));
+              const float2 e2 = f2_unpack(f2_mul(f2_add(f2_pack(F1[u].x, F1[u].y), q2), iw2));
+              const float2 e3 = f2_unpack(f2_mul(f2_sub(f2_pack(F1[u].z, F1[u].w), q3), iw3));
+              const unsigned long long r = f2_mul(f2_pack(F3.x, F3.y), gfac);
+              const float2 tv = f2_unpack(t), t2 = f2_unpack(f2_mul(t, t));
               const unsigned long long rtt =
                   f2_mul(r, f2_pack(tv.x > 0.1f ? t2.x : 0.01f, tv.y > 0.1f ? t2.y : 0.01f));
               const float2 den = f2_unpack(f2_mul(uz, rtt));
-              const unsigned long long inv =
-                  f2_pack(__fdividef(1.0f, den.x), __fdividef(1.0f, den.y));
+              const unsigned long long inv = f2_pack(rcp_fast(den.x), rcp_fast(den.y));
               const unsigned long long ruz = f2_mul(rtt, inv);
-              const float2 exr = f2_unpack(f2_mul(f2_pack(fminf(ex1.x, ex2.x), fminf(ex1.y, ex2.y)), ruz));
-              const float2 eyr = f2_unpack(f2_mul(f2_pack(fminf(ey1.x, ey2.x), fminf(ey1.y, ey2.y)), ruz));
-              const unsigned long long wt = f2_mul(f2_pack(fminf(1.0f, exr.x), fminf(1.0f, exr.y)),
-                                                   f2_pack(fminf(1.0f, eyr.x), fminf(1.0f, eyr.y)));
-              unsigned long long fac = f2_mul(f2_mul(wt, f2_fma(r, r, f2_pack(1.0f, 1.0f))),
-                                              f2_mul(f2_mul(f2_pack(100.0f, 100.0f), uz), inv));
-              if (std::is_same<T, __half>::value)  // 2^e from the records' exponent bits
-                fac = f2_mul(fac, f2_pack(
-                    __int_as_float((int)((((unsigned)rec[0].y >> 24) - 1u) << 23)),
-                    __int_as_float((int)((((unsigned)rec[1].y >> 24) - 1u) << 23))));
-              // samples (index clamped into the panel; loads only for imaged members)
-              const T *q0 = panels + (size_t)rec[0].x * pstride +
-                            (unsigned)(b00 * a.nt + min(max(it0, 0), a.nt - 2));
-              const T *q1 = panels + (size_t)rec[1].x * pstride +
-                            (unsigned)(b01 * a.nt + min(max(it1v, 0), a.nt - 2));
-              float s00 = 0.f, s01 = 0.f, s10 = 0.f, s11 = 0.f;
-              float u00 = 0.f, u01 = 0.f, u10 = 0.f, u11 = 0.f;
-              if (on[0]) {
-                s00 = ld_sample<T>(q0);
-                s01 = ld_sample<T>(q0 + 1);
-                s10 = ld_sample<T>(q0 + a.nt);
-                s11 = ld_sample<T>(q0 + a.nt + 1);
-              }
-              if (on[1]) {
-                u00 = ld_sample<T>(q1);
-                u01 = ld_sample<T>(q1 + 1);
-                u10 = ld_sample<T>(q1 + a.nt);
-                u11 = ld_sample<T>(q1 + a.nt + 1);
-              }
-              const unsigned long long p00 = f2_pack(s00, u00), p01 = f2_pack(s01, u01);
-              const unsigned long long p10 = f2_pack(s10, u10), p11 = f2_pack(s11, u11);
-              const unsigned long long sa = f2_fma(fwt, f2_sub(p01, p00), p00);
-              const unsigned long long sb = f2_fma(fwt, f2_sub(p11, p10), p10);
-              const float2 v = f2_unpack(f2_mul(fac, f2_fma(fwb, f2_sub(sb, sa), sa)));
+              const float2 ex =
+                  f2_unpack(f2_mul(f2_pack(fminf(e0.x, e1.x), fminf(e0.y, e1.y)), ruz));
+              const float2 ey =
+                  f2_unpack(f2_mul(f2_pack(fminf(e2.x, e3.x), fminf(e2.y, e3.y)), ruz));
+              const unsigned long long wt = f2_mul(f2_pack(fminf(1.0f, ex.x), fminf(1.0f, ex.y)),
+                                                   f2_pack(fminf(1.0f, ey.x), fminf(1.0f, ey.y)));
+              const float2 fv = f2_unpack(
+                  f2_mul(f2_mul(wt, f2_fma(r, r, f2_dup(1.0f))),
+                         f2_mul(f2_mul(f2_dup(__int_as_float(rec[u].w)), uz), inv)));
+              fac[u] = f2_pack(on[u][0] ? fv.x : 0.0f, on[u][1] ? fv.y : 0.0f);
+              cimg += on[u][0];
+              cimg += on[u][1];
+            }
+            float sm[U][2][4];
 #pragma unroll
-              for (int u = 0; u < 2; ++u) {
-                if (!on[u]) continue;
-                ++cimg;
-                const float vu = u ? v.y : v.x;
-                if (comp) {
-                  const float y = vu - cmp;
-                  const float tt = acc + y;
-                  cmp = (tt - acc) - y;
-                  acc = tt;
-                } else {
-                  acc += vu;
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+              for (int p = 0; p < 2; ++p) {
+                sm[u][p][0] = sm[u][p][1] = sm[u][p][2] = sm[u][p][3] = 0.0f;
+                if (on[u][p]) {
+                  const T *q = pp[u][p];
+                  sm[u][p][0] = ld_sample<T>(q);
+                  sm[u][p][1] = ld_sample<T>(q + 1);
+                  sm[u][p][2] = ld_sample<T>(q + a.nt);
+                  sm[u][p][3] = ld_sample<T>(q + a.nt + 1);
                 }
               }
-              continue;
-            }
-            bool on[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-              const int lo = rec[u].z >> 16, hi = rec[u].z & 0xFFFF;
-              const bool inr = val[u] && (unsigned)(lx - lo) <= (unsigned)(hi - lo);
-              const float4 B = planeB[(size_t)(rec[u].y & 0xFF) * NT + tid];
-              on[u] = inr && B.x > qx1 && B.y > qx2 && B.z > qy1 && B.w > qy2;
-            }
-            const T *pp[U];
-            float fwt[U], fwb[U], fac[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-              pp[u] = panels;
-              fwt[u] = fwb[u] = fac[u] = 0.0f;
-              if (!on[u]) continue;
-              on[u] = false;
-              const float4 A = planeA[(size_t)(rec[u].y & 0xFF) * NT + tid];
-              const float4 B = planeB[(size_t)(rec[u].y & 0xFF) * NT + tid];
-              const float uz = A.w + agz;
-              const float ex = fminf((B.x - qx1) * iwx1, (B.y - qx2) * iwx2);
-              const float ey = fminf((B.z - qy1) * iwy1, (B.w - qy2) * iwy2);
-              const float t = A.x + tg;
-              const float ft = t * inv_dt1;
-              const int it1 = (int)ft;
-              if (!(it1 > 0 && it1 + 1 < a.nt)) continue;
-              const float fb = fminf(fmaxf(A.y + qg, 0.0f), (float)(a.nbins - 1));
-              const int b0 = min((int)fb, a.nbins - 2);
-              fwt[u] = ft - (float)it1;
-              fwb[u] = fb - (float)b0;
-              pp[u] = panels + (size_t)rec[u].x * pstride + (unsigned)(b0 * a.nt + it1);
-              // w v (r + 1/r) = w (r^2 + 1) 100 / (r tt), tt = t^2 (0.01 below 0.1 s)
-              const float r = A.z * gfac;
-              const float rtt = r * (t > 0.1f ? t * t : 0.01f);
-              const float inv = __fdividef(1.0f, uz * rtt);
-              const float ruz = rtt * inv;
-              const float wt = fminf(1.0f, ex * ruz) * fminf(1.0f, ey * ruz);
-              fac[u] = wt * fmaf(r, r, 1.0f) * (100.0f * uz * inv);
-              if (std::is_same<T, __half>::value)  // 2^e from the record's exponent bits
-                fac[u] *= __int_as_float((int)((((unsigned)rec[u].y >> 24) - 1u) << 23));
-              on[u] = true;
-              ++cimg;
-            }
-            float smp[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-              smp[u] = 0.0f;
-              if (on[u]) {
-                const T *q = pp[u];
-                const float p00 = ld_sample<T>(q), p01 = ld_sample<T>(q + 1);
-                const float p10 = ld_sample<T>(q + a.nt), p11 = ld_sample<T>(q + a.nt + 1);
-                const float s0v = p00 + fwt[u] * (p01 - p00), s1v = p10 + fwt[u] * (p11 - p10);
-                smp[u] = s0v + fwb[u] * (s1v - s0v);
-              }
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-              if (!on[u]) continue;
-              const float v = fac[u] * smp[u];
-              if (comp) {
-                const float y = v - cmp;
-                const float tt = acc + y;
-                cmp = (tt - acc) - y;
+              const unsigned long long p00 = f2_pack(sm[u][0][0], sm[u][1][0]);
+              const unsigned long long p01 = f2_pack(sm[u][0][1], sm[u][1][1]);
+              const unsigned long long p10 = f2_pack(sm[u][0][2], sm[u][1][2]);
+              const unsigned long long p11 = f2_pack(sm[u][0][3], sm[u][1][3]);
+              const unsigned long long v = f2_lerp(f2_lerp(p00, p01, fwt[u]),
+                                                   f2_lerp(p10, p11, fwt[u]), fwb[u]);
+              if (comp) {  // Kahan-compensated sums (a point that is off adds zero)
+                const unsigned long long y = f2_sub(f2_mul(fac[u], v), cmp);
+                const unsigned long long tt = f2_add(acc, y);
+                cmp = f2_sub(f2_sub(tt, acc), y);
                 acc = tt;
               } else {
-                acc += v;
+                acc = f2_fma(fac[u], v, acc);
               }
             }
           }
         }
-        __syncthreads();  // s_mask, s_wpos and s_list are rewritten by the next chunk
+        __syncthreads();  // s_mask, s_wpos, s_rec and s_geo are rewritten by the next chunk
       }
     }
-    if (live) {
-      img[(size_t)ixb * a.nzi + izi] = acc;
-      if (comp) comp[(size_t)ixb * a.nzi + izi] = cmp;
+    const float2 av = f2_unpack(acc), cv = f2_unpack(cmp);
+    const size_t o = (size_t)ixb * a.nzi + izi;
+    if (nsplit == 1) {
+#pragma unroll
+      for (int p = 0; p < 2; ++p)
+        if (live[p]) {
+          img[o + p] = p ? av.y : av.x;
+          if (comp) comp[o + p] = p ? cv.y : cv.x;
+        }
+      continue;
     }
+    const size_t nimg = (size_t)a.nxb * a.nzi;
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+      if (live[p]) part[ipart * nimg + o + p] = (p ? av.y : av.x) - (p ? cv.y : cv.x);
+    if (!last_part(tile_done + tile, nsplit, &s_tile)) continue;
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+      if (live[p])
+        add_parts(img + o + p, comp ? comp + o + p : nullptr, part + o + p, nimg, nsplit);
   }
   if (npt) add_counts(npt, s_cnt, cnt, cdrop, cimg);
 }
@@ -2026,8 +2256,6 @@ static int batched_alloc(PhysicsState *s, const qpsdm_static_params &p) {
     ok &= cudaMalloc(&g.d_mem, sizeof(int4) * n) == cudaSuccess;
     ok &= cudaMalloc(&g.d_grppos, sizeof(float2) * n) == cudaSuccess;
     ok &= cudaMalloc(&g.d_memgrp, sizeof(int) * n) == cudaSuccess;
-    ok &= cudaMalloc(&g.d_tile_ctr, sizeof(int)) == cudaSuccess;
-    ok &= cudaMalloc(&g.d_ndefer, sizeof(int)) == cudaSuccess;
     ok &= cudaMalloc(&g.d_nmem, sizeof(int)) == cudaSuccess;
   }
   if (!ok) return QPSDM_ENOMEM;
@@ -2077,23 +2305,42 @@ struct LineView {
 // the extra loads in flight gain.)
 // Variants from 13 on are the fast form (k_image_batched_fast, with
 // k_image_batched over the tiles it leaves) with mw words of 32 members per
-// chunk; cl = 2: the walk on packed FP32 pairs.
+// chunk.  16 x 16 tiles of 128 threads at 96 registers (five CTAs, 20 warps
+// an SM) win wherever images are large: against 64-thread tiles the keep pass
+// and the chunk's barriers serve twice the points, against 128 registers the
+// fourth warp per scheduler hides more of the panel loads than the spilled
+// words cost.
 struct BatchedVariant {
-  int tz, tx, mb, sc, u, cl, mw;
+  int tz, tx, mb, sc, u, mw;
 };
 static const BatchedVariant kVariants[] = {
-    {32, 8, 2, 8, 4, 0, 0},   {32, 4, 4, 8, 4, 0, 0},   {32, 4, 6, 8, 4, 0, 0},
-    {64, 4, 3, 8, 4, 0, 0},   {32, 4, 3, 16, 4, 0, 0},  {8, 16, 4, 8, 4, 0, 0},
-    {4, 32, 4, 8, 4, 0, 0},   {16, 8, 4, 8, 4, 0, 0},   {8, 16, 4, 16, 4, 0, 0},
-    {16, 8, 3, 16, 4, 0, 0},  {8, 16, 5, 8, 4, 0, 0},   {8, 16, 5, 16, 4, 0, 0},
-    {16, 8, 5, 8, 4, 0, 0},   {8, 16, 5, 8, 4, 1, 16},  {8, 16, 4, 8, 4, 1, 32},
-    {16, 8, 5, 8, 4, 1, 16},  {32, 4, 5, 8, 4, 1, 16},  {8, 16, 4, 16, 4, 1, 16},
-    {16, 8, 4, 8, 4, 1, 32},  {8, 16, 6, 8, 2, 1, 8},   {8, 16, 6, 8, 4, 1, 8},
-    {16, 8, 6, 8, 2, 1, 8},   {8, 16, 5, 8, 2, 1, 16},  {8, 16, 6, 8, 2, 2, 8},
-    {8, 16, 5, 8, 2, 2, 8},
+    {32, 8, 2, 8, 4, 0},  {32, 4, 4, 8, 4, 0},  {32, 4, 6, 8, 4, 0},
+    {64, 4, 3, 8, 4, 0},  {32, 4, 3, 16, 4, 0}, {8, 16, 4, 8, 4, 0},
+    {4, 32, 4, 8, 4, 0},  {16, 8, 4, 8, 4, 0},  {8, 16, 4, 16, 4, 0},
+    {16, 8, 3, 16, 4, 0}, {8, 16, 5, 8, 4, 0},  {8, 16, 5, 16, 4, 0},
+    {16, 8, 5, 8, 4, 0},  {8, 16, 8, 4, 1, 8},  {8, 16, 8, 4, 2, 8},
+    {16, 8, 8, 4, 2, 8},  {32, 4, 8, 4, 2, 8},  {8, 16, 5, 8, 2, 8},
+    {16, 8, 5, 8, 2, 8},  {8, 16, 10, 4, 1, 8}, {8, 16, 5, 8, 1, 8},
+    {16, 8, 10, 4, 1, 8}, {8, 16, 6, 4, 2, 8},  {8, 16, 8, 2, 2, 8},
+    {8, 16, 8, 4, 2, 16}, {16, 16, 5, 4, 1, 8}, {16, 16, 4, 4, 1, 8},
 };
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 static_assert(kNumVariants <= 32, "tune_ms holds 32 timings");
+
+// Parts of a tile's members for an image of ntiles tiles: 32 queue items per
+// SM, of at least 64 members each, as far as the sums have room.  Tiles differ
+// in work by an order of magnitude (the middle of the aperture keeps most
+// members, its rim few), so one item per tile leaves most SMs waiting for a
+// few: a 512 x 400 line of 18,432 traces (800 tiles of 16 x 16) took 6.3 ms
+// in one part per tile, the SMs active 60 % of the time, and 3.1 ms in six;
+// 16, 48 and 128 items per SM were no faster.  A 128 x 100 line of 1,024
+// traces: 1.29 ms unsplit, 0.08 ms split.  An image of more tiles than that
+// is not split (1024 x 600: 2,432 tiles, 38.1 ms against 38.3 for eight lines).
+static int member_split(const PhysicsState *s, const PhysImageArgs &a, int ntiles, int ntr) {
+  const int want = (32 * s->num_sms + ntiles - 1) / ntiles;
+  const size_t room = s->part_cap / ((size_t)a.nxb * a.nzi);
+  return std::max(1, std::min(std::min(want, ntr / 64), std::min((int)room, kMaxSplit)));
+}
 
 // The original kernel over every tile of the image, or (tile_list) over the
 // *ntile_list tiles of a list, with one persistent CTA per SM.
@@ -2103,7 +2350,7 @@ static int launch_batched_tile(PhysicsState *s, const PhysImageArgs &a, const Ph
                                unsigned long long *npt, int sc, cudaStream_t st,
                                const int *tile_list = nullptr,
                                const int *ntile_list = nullptr) {
-  const int ntz = (a.nzi + TZ - 1) / TZ, ntx = (a.nxb + TX - 1) / TX;
+  const int ntz = (a.nzi + TZ - 1) / TZ, ntx = (a.nxb + TX - 1) / TX, ntiles = ntz * ntx;
   const size_t smem = sizeof(float2) * kMapN * (size_t)sc * TZ * TX;
   auto kern = k_image_batched<TZ, TX, MB, U, T>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
@@ -2111,44 +2358,59 @@ static int launch_batched_tile(PhysicsState *s, const PhysImageArgs &a, const Ph
     return QPSDM_ECUDA;
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TZ * TX, smem);
-  const int grid = tile_list ? std::max(1, s->num_sms)
-                             : std::max(1, std::min(ntz * ntx, std::max(per_sm, 1) * s->num_sms));
-  cudaMemsetAsync(s->d_tile_ctr, 0, sizeof(int), st);
+  const int nsplit = member_split(s, a, ntiles, b.ntr);
+  const int grid =
+      tile_list ? std::max(1, s->num_sms)
+                : std::max(1, std::min(ntiles * nsplit, std::max(per_sm, 1) * s->num_sms));
+  // the queue's counter and, unless the tiles come from the fast form's list
+  // (which has cleared them), the finished parts
+  cudaMemsetAsync(s->d_tile_ctr, 0,
+                  sizeof(int) * (size_t)(!tile_list && nsplit > 1 ? 2 + ntiles : 1), st);
   kern<<<grid, TZ * TX, smem, st>>>(img, comp, a, v.dips, s->d_memgrp, s->d_grppos, s->d_mem,
                                     s->d_nmem, s->d_srcpos, s->d_sid + (b.ntr - 1), v.tab->dt,
                                     v.tab->ttt, v.tab->dq, v.tab->qqq,
                                     v.tab->paired ? v.tab->tq : nullptr, (const T *)s->d_panels,
-                                    s->d_tile_ctr, ntz, ntx, sc, npt, tile_list, ntile_list);
+                                    s->d_tile_ctr, ntz, ntx, sc, npt, tile_list, ntile_list,
+                                    nsplit, s->d_part, s->d_tile_ctr + 2);
   return cudaGetLastError() == cudaSuccess ? QPSDM_OK : QPSDM_ECUDA;
+}
+
+// Whether every tile of the image is uniform (k_image_batched_fast leaves
+// none): one depth cell, one surface grid, and tile columns that do not
+// straddle the tables' x-cells.
+static bool all_uniform(const PhysImageArgs &a, const PhysicsState::LineTab &t, int tx) {
+  return t.one_grid && a.nzg == 1 && a.nxi1 % tx == 0 && (a.ixstart - a.tcdp1) % tx == 0;
 }
 
 // The fast form over the image's uniform tiles, then the original kernel
 // (same tile shape, MBO blocks per SM) over the tiles it left; with unpaired
 // tables the original kernel takes every tile.
-template <int TZ, int TX, int MB, int U, int MW, int MBO, typename T, bool PK = false>
+template <int TZ, int TX, int MB, int U, int MW, int MBO, typename T>
 static int launch_batched_fast(PhysicsState *s, const PhysImageArgs &a, const PhysicsBatch &b,
                                const LineView &v, float *img, float *comp,
                                unsigned long long *npt, int sc, cudaStream_t st) {
   if (!v.tab->paired)
     return launch_batched_tile<TZ, TX, MBO, 4, T>(s, a, b, v, img, comp, npt, sc, st);
-  const int ntz = (a.nzi + TZ - 1) / TZ, ntx = (a.nxb + TX - 1) / TX;
-  if ((size_t)ntz * ntx > s->defer_cap) return QPSDM_EINVAL;  // cannot happen: sized per offset
+  const int ntz = (a.nzi + TZ - 1) / TZ, ntx = (a.nxb + TX - 1) / TX, ntiles = ntz * ntx;
+  if ((size_t)ntiles > s->defer_cap) return QPSDM_EINVAL;  // cannot happen: sized per offset
   const size_t smem = sizeof(float4) * 2 * (size_t)sc * TZ * TX;
-  auto kern = k_image_batched_fast<TZ, TX, MB, U, MW, PK, T>;
+  auto kern = k_image_batched_fast<TZ, TX, MB, U, MW, T>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return QPSDM_ECUDA;
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TZ * TX, smem);
-  const int grid = std::max(1, std::min(ntz * ntx, std::max(per_sm, 1) * s->num_sms));
-  cudaMemsetAsync(s->d_tile_ctr, 0, sizeof(int), st);
-  cudaMemsetAsync(s->d_ndefer, 0, sizeof(int), st);
-  kern<<<grid, TZ * TX, smem, st>>>(img, comp, a, v.dips, s->d_memgrp, s->d_grppos, s->d_mem,
-                                    s->d_nmem, s->d_srcpos, s->d_sid + (b.ntr - 1), v.tab->dt,
-                                    v.tab->ttt, v.tab->dq, v.tab->qqq, v.tab->tq,
-                                    (const T *)s->d_panels, s->d_tile_ctr, ntz, ntx, sc, npt,
-                                    s->d_defer, s->d_ndefer);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TZ * TX / 2, smem);
+  const int nsplit = member_split(s, a, ntiles, b.ntr);
+  const int grid = std::max(1, std::min(ntiles * nsplit, std::max(per_sm, 1) * s->num_sms));
+  // queue counter, deferred-tile count and the split tiles' finished parts
+  cudaMemsetAsync(s->d_tile_ctr, 0, sizeof(int) * (size_t)(nsplit > 1 ? 2 + ntiles : 2), st);
+  kern<<<grid, TZ * TX / 2, smem, st>>>(
+      img, comp, a, v.dips, s->d_memgrp, s->d_grppos, s->d_mem, s->d_nmem, s->d_srcpos,
+      s->d_sid + (b.ntr - 1), v.tab->dt, v.tab->dq, v.tab->tq, (const T *)s->d_panels,
+      s->d_tile_ctr, ntz, ntx, sc, npt, s->d_defer, s->d_ndefer, nsplit, s->d_part,
+      s->d_tile_ctr + 2);
   if (cudaGetLastError() != cudaSuccess) return QPSDM_ECUDA;
+  if (all_uniform(a, *v.tab, TX)) return QPSDM_OK;
   return launch_batched_tile<TZ, TX, MBO, 4, T>(s, a, b, v, img, comp, npt, sc, st, s->d_defer,
                                                 s->d_ndefer);
 }
@@ -2159,18 +2421,20 @@ static int launch_variant(int vi, PhysicsState *s, const PhysImageArgs &a, const
                           cudaStream_t st) {
   const int sc = kVariants[vi].sc;
   switch (vi) {
-    case 13: return launch_batched_fast<8, 16, 5, 4, 16, 4, T>(s, a, b, v, img, comp, npt, sc, st);
-    case 14: return launch_batched_fast<8, 16, 4, 4, 32, 4, T>(s, a, b, v, img, comp, npt, sc, st);
-    case 15: return launch_batched_fast<16, 8, 5, 4, 16, 4, T>(s, a, b, v, img, comp, npt, sc, st);
-    case 16: return launch_batched_fast<32, 4, 5, 4, 16, 4, T>(s, a, b, v, img, comp, npt, sc, st);
-    case 17: return launch_batched_fast<8, 16, 4, 4, 16, 4, T>(s, a, b, v, img, comp, npt, sc, st);
-    case 18: return launch_batched_fast<16, 8, 4, 4, 32, 4, T>(s, a, b, v, img, comp, npt, sc, st);
-    case 19: return launch_batched_fast<8, 16, 6, 2, 8, 4, T>(s, a, b, v, img, comp, npt, sc, st);
-    case 20: return launch_batched_fast<8, 16, 6, 4, 8, 4, T>(s, a, b, v, img, comp, npt, sc, st);
-    case 21: return launch_batched_fast<16, 8, 6, 2, 8, 4, T>(s, a, b, v, img, comp, npt, sc, st);
-    case 22: return launch_batched_fast<8, 16, 5, 2, 16, 4, T>(s, a, b, v, img, comp, npt, sc, st);
-    case 23: return launch_batched_fast<8, 16, 6, 2, 8, 4, T, true>(s, a, b, v, img, comp, npt, sc, st);
-    case 24: return launch_batched_fast<8, 16, 5, 2, 8, 4, T, true>(s, a, b, v, img, comp, npt, sc, st);
+    case 13: return launch_batched_fast<8, 16, 8, 1, 8, 4, T>(s, a, b, v, img, comp, npt, sc, st);
+    case 14:
+    case 23: return launch_batched_fast<8, 16, 8, 2, 8, 4, T>(s, a, b, v, img, comp, npt, sc, st);
+    case 15: return launch_batched_fast<16, 8, 8, 2, 8, 4, T>(s, a, b, v, img, comp, npt, sc, st);
+    case 16: return launch_batched_fast<32, 4, 8, 2, 8, 4, T>(s, a, b, v, img, comp, npt, sc, st);
+    case 17: return launch_batched_fast<8, 16, 5, 2, 8, 4, T>(s, a, b, v, img, comp, npt, sc, st);
+    case 18: return launch_batched_fast<16, 8, 5, 2, 8, 4, T>(s, a, b, v, img, comp, npt, sc, st);
+    case 19: return launch_batched_fast<8, 16, 10, 1, 8, 4, T>(s, a, b, v, img, comp, npt, sc, st);
+    case 20: return launch_batched_fast<8, 16, 5, 1, 8, 4, T>(s, a, b, v, img, comp, npt, sc, st);
+    case 21: return launch_batched_fast<16, 8, 10, 1, 8, 4, T>(s, a, b, v, img, comp, npt, sc, st);
+    case 22: return launch_batched_fast<8, 16, 6, 2, 8, 4, T>(s, a, b, v, img, comp, npt, sc, st);
+    case 24: return launch_batched_fast<8, 16, 8, 2, 16, 4, T>(s, a, b, v, img, comp, npt, sc, st);
+    case 25: return launch_batched_fast<16, 16, 5, 1, 8, 2, T>(s, a, b, v, img, comp, npt, sc, st);
+    case 26: return launch_batched_fast<16, 16, 4, 1, 8, 2, T>(s, a, b, v, img, comp, npt, sc, st);
     case 0: return launch_batched_tile<32, 8, 2, 4, T>(s, a, b, v, img, comp, npt, sc, st);
     case 1: return launch_batched_tile<32, 4, 4, 4, T>(s, a, b, v, img, comp, npt, sc, st);
     case 2: return launch_batched_tile<32, 4, 6, 4, T>(s, a, b, v, img, comp, npt, sc, st);
