@@ -119,7 +119,8 @@ int launch_gate(const uint8_t *d_rec, int rec_bytes, int ntr, int be,
 }
 
 // ---------------------------------------------------------------------------
-// Spectra: one CTA per (accepted trace, window).
+// Spectra: one CTA per accepted trace, its two windows transformed together
+// (fft.cuh).
 // ---------------------------------------------------------------------------
 
 // Gained sample j of the trace, then the full-trace end taper applied in the
@@ -151,38 +152,45 @@ __device__ __forceinline__ float gained(float v, int it, float dt) {
   return __fmul_rn(v, __fmul_rn(t, t));
 }
 
-__global__ void __launch_bounds__(256) k_spectra(const uint8_t *__restrict__ rec,
-                                                 int rec_bytes, int be,
-                                                 const int *__restrict__ ints,
-                                                 SpectraArgs a, FftPlan p,
-                                                 float *__restrict__ re,
-                                                 float *__restrict__ im) {
-  const int itr = blockIdx.x, win = blockIdx.y;
+// Sample i of window [itb, itb + nsb) of the trace, tapered again to the window.
+__device__ __forceinline__ float window_sample(const uint8_t *r, int be, const SpectraArgs &a,
+                                               int itb, int i) {
+  const int j = itb + i;
+  float v = 0.0f;
+  if (j >= 0 && j < a.ntl)
+    v = tapered_sample(gained(su_sample(r, j, be), j, a.dt), j, a.ntl, a.taper200);
+  return tapered_sample(v, i, a.nsb, a.taper200);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kFftMaxThreads, 2)
+    k_spectra(const uint8_t *__restrict__ rec, int rec_bytes, int be,
+              const int *__restrict__ ints, const __grid_constant__ SpectraArgs a,
+              const __grid_constant__ FftPlan p, float *__restrict__ re,
+              float *__restrict__ im) {
+  const int itr = blockIdx.x;
   if (ints[(size_t)itr * kGateInts] != kAccepted) return;
-  extern __shared__ float2 sm[];
-  float2 *b0 = sm, *b1 = sm + p.m, *twm = sm + 2 * p.m, *twn = sm + 3 * p.m;
-  for (int i = threadIdx.x; i < p.m; i += blockDim.x) twm[i] = p.tw_m[i];
-  for (int i = threadIdx.x; i <= p.m; i += blockDim.x) twn[i] = p.tw_n[i];
+  extern __shared__ float4 pbuf[];
   const uint8_t *r = rec + (size_t)itr * rec_bytes;
-  const int itb = win == 0 ? a.itb1 : a.itb2;
-  float *bf = reinterpret_cast<float *>(b0);
-  for (int i = threadIdx.x; i < a.nsb; i += blockDim.x) {
-    const int j = itb + i;
-    float v = 0.0f;
-    if (j >= 0 && j < a.ntl)
-      v = tapered_sample(gained(su_sample(r, j, be), j, a.dt), j, a.ntl, a.taper200);
-    bf[i] = tapered_sample(v, i, a.nsb, a.taper200);
-  }
+  for (int j = threadIdx.x; j < p.m; j += blockDim.x)
+    pbuf[pfa_slot<MODE>(j)] = make_float4(
+        window_sample(r, be, a, a.itb1, 2 * j), window_sample(r, be, a, a.itb2, 2 * j),
+        window_sample(r, be, a, a.itb1, 2 * j + 1), window_sample(r, be, a, a.itb2, 2 * j + 1));
   __syncthreads();
-  const int cur = fft_complex_smem(b0, b1, p, twm, false);
-  const float2 *Z = cur ? b1 : b0;
-  float *ro = re + (size_t)itr * 2 * a.nww + win * a.nww;
-  float *io = im + (size_t)itr * 2 * a.nww + win * a.nww;
+  const float4 *Z = fft_passes<MODE>(pbuf, p);
+  float *ro = re + (size_t)itr * 2 * a.nww, *io = im + (size_t)itr * 2 * a.nww;
   for (int iw = threadIdx.x; iw < a.nww; iw += blockDim.x) {
-    const float2 X = rfft_bin(Z, twn, p.m, iw + a.nf1);
+    // bin k <= m from Z[k] and Z[m-k]
+    const int k = iw + a.nf1;
+    C2 X, unused;
+    pfa_rfft_bins(pfa_ld(Z, pfa_slot<MODE>(k == p.m ? 0 : k)),
+                  pfa_ld(Z, pfa_slot<MODE>(k == 0 ? 0 : p.m - k)), __ldg(p.tw_n + k), X, unused);
+    const float2 xr = f2_unpack(X.re), xi = f2_unpack(X.im);
     const float w = a.omega[iw];
-    ro[iw] = __fmul_rn(X.y, w);
-    io[iw] = -__fmul_rn(X.x, w);
+    ro[iw] = __fmul_rn(xi.x, w);
+    io[iw] = -__fmul_rn(xr.x, w);
+    ro[a.nww + iw] = __fmul_rn(xi.y, w);
+    io[a.nww + iw] = -__fmul_rn(xr.y, w);
   }
 }
 
@@ -194,10 +202,13 @@ int launch_spectra(const uint8_t *d_rec, int rec_bytes, int ntr, int be,
   std::string err;
   int rc = fft_plan(a.nsb, &p, &err);
   if (rc) return rc;
-  const size_t sm = fft_smem_bytes(p.m);
-  if ((rc = fft_set_smem_attr((const void *)k_spectra, sm))) return rc;
-  k_spectra<<<dim3(ntr, 2), 256, sm, s>>>(d_rec, rec_bytes, be, d_ints, a, p, d_re, d_im);
-  return cudaGetLastError() == cudaSuccess ? QPSDM_OK : QPSDM_ECUDA;
+  return fft_by_mode(p, [&](auto mode) {
+    auto kern = k_spectra<decltype(mode)::value>;
+    const size_t sm = fft_smem_bytes(p);
+    if ((rc = fft_set_smem_attr((const void *)kern, sm))) return rc;
+    kern<<<ntr, p.threads, sm, s>>>(d_rec, rec_bytes, be, d_ints, a, p, d_re, d_im);
+    return cudaGetLastError() == cudaSuccess ? (int)QPSDM_OK : (int)QPSDM_ECUDA;
+  });
 }
 
 // ---------------------------------------------------------------------------

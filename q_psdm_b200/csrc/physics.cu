@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "f32x2.cuh"
 #include "fft.cuh"
 #include "internal.h"
 #include "physics.h"
@@ -72,7 +73,8 @@ constexpr size_t kSplitSums = 1 << 23;
 struct PhysicsState {
   int nfft = 0, nffti = 0, nbins = 0, max_batch = 0, dtype = 0;
   float dtstar = 0.0f;
-  float2 *d_filter = nullptr;  // [nbins][nfft/2+1]
+  float4 *d_filter = nullptr;  // [(nbins+1)/2][kmax]: (re, re, im, im) of two bins
+  int kmax = 0;                // first frequency bin past the band
   float2 *d_spec = nullptr;    // [max_batch][nfft/2+1]
   float *d_fmax = nullptr;     // [nfft/2+1] max over bins of |filter|
   float *d_pscale = nullptr;   // [max_batch] FP16 panels: per-trace sample multiplier
@@ -161,9 +163,10 @@ static void select_set(PhysicsState *s, int i) {
 static size_t dtype_bytes(int t) { return t == QPSDM_PANEL_FP32 ? 4 : 2; }
 static int batched_alloc(PhysicsState *s, const qpsdm_static_params &p);
 
-// (-i ww_k) * A(pi f t*) * exp(-2 i f t* ln(f/fc)) / nfft for every bin.
+// (-i ww_k) * A(pi f t*) * exp(-2 i f t* ln(f/fc)) / nfft for every bin, and
+// the first frequency bin past the band.
 static void filter_table(const qpsdm_static_params &p, int nbins, float dtstar,
-                         std::vector<float2> &out, std::vector<float> &fmax) {
+                         std::vector<float2> &out, std::vector<float> &fmax, int *kmax) {
   const int nk = p.nfft / 2 + 1;
   const double df = 1.0 / ((double)p.nfft * (double)p.dt);
   const double dw = 2.0 * M_PI * df;
@@ -172,6 +175,7 @@ static void filter_table(const qpsdm_static_params &p, int nbins, float dtstar,
   const double c1 = G * (1.0 - lnG - 2.5 * lnG * lnG), c2 = G * (1.0 + 5.0 * lnG);
   const double c3 = -2.5 * G, c4 = 1.1 * G;
   out.assign((size_t)nbins * nk, make_float2(0.f, 0.f));
+  *kmax = std::max(1, std::min(nk, n4));
   for (int b = 0; b < nbins; ++b) {
     const double ts = b * (double)dtstar;
     for (int k = 1; k < nk; ++k) {
@@ -229,15 +233,22 @@ int physics_create(PhysicsState **out, const qpsdm_static_params &p, std::string
   s->dtype = p.panel_dtype;
   std::vector<float2> f;
   std::vector<float> fmax;
-  filter_table(p, p.nbins, p.dtstar, f, fmax);
+  filter_table(p, p.nbins, p.dtstar, f, fmax, &s->kmax);
   const size_t nk = (size_t)p.nfft / 2 + 1;
   auto bad = [&](const char *w) {
     if (err) *err = std::string("physics_create: ") + w;
     physics_destroy(s);
     return QPSDM_ENOMEM;
   };
-  if (cudaMalloc(&s->d_filter, sizeof(float2) * f.size()) != cudaSuccess) return bad("filter");
-  cudaMemcpy(s->d_filter, f.data(), sizeof(float2) * f.size(), cudaMemcpyHostToDevice);
+  std::vector<float4> pairs((size_t)(p.nbins + 1) / 2 * s->kmax, make_float4(0.f, 0.f, 0.f, 0.f));
+  for (int q = 0; q < p.nbins; ++q)
+    for (int k = 0; k < s->kmax; ++k) {
+      float *d = &pairs[(size_t)(q / 2) * s->kmax + k].x;
+      d[q & 1] = f[q * nk + k].x;
+      d[2 + (q & 1)] = f[q * nk + k].y;
+    }
+  if (cudaMalloc(&s->d_filter, sizeof(float4) * pairs.size()) != cudaSuccess) return bad("filter");
+  cudaMemcpy(s->d_filter, pairs.data(), sizeof(float4) * pairs.size(), cudaMemcpyHostToDevice);
   if (cudaMalloc(&s->d_spec, sizeof(float2) * nk * p.max_batch) != cudaSuccess) return bad("spectra");
   if (cudaMalloc(&s->d_fmax, sizeof(float) * nk) != cudaSuccess) return bad("filter bound");
   cudaMemcpy(s->d_fmax, fmax.data(), sizeof(float) * nk, cudaMemcpyHostToDevice);
@@ -537,175 +548,206 @@ __device__ __forceinline__ float phys_tapered(float v, int j, int n, const float
   return v;
 }
 
-// Forward spectra of the accepted traces; a persistent CTA loads the
-// twiddles into shared memory once and then takes every gridDim.x-th trace.
-// For FP16 panels also the trace's sample multiplier: every panel sample of
-// the trace is bounded by B = 2 sum_k |X_k| max_b |F_b,k| (triangle
+// Gained and tapered sample j of a trace (zero beyond its end).
+__device__ __forceinline__ float phys_sample(const uint8_t *r, int j, int be, int ntl, float dt,
+                                             const float *tap) {
+  if (j >= ntl) return 0.0f;
+  float v = su_sample(r, j, be);
+  const float t = __fmul_rn((float)j, dt);
+  v = ((double)t < 0.1) ? __double2float_rn(__dmul_rn((double)v, 0.1 * 0.1))
+                        : __fmul_rn(v, __fmul_rn(t, t));
+  return phys_tapered(v, j, ntl, tap);
+}
+
+// Forward spectra of the accepted traces, two neighbouring traces per CTA
+// (fft.cuh).  For FP16 panels also the trace's sample multiplier: every panel
+// sample of the trace is bounded by B = 2 sum_k |X_k| max_b |F_b,k| (triangle
 // inequality over the c2r sum), and the panels store x / 2^e with e chosen so
 // that B / 2^e lies in [2^13, 2^14): no overflow of FP16 (max 65504) and no
 // loss to its subnormal range; the image kernels multiply the samples by 2^e
 // again (exact).
-__global__ void __launch_bounds__(256) k_phys_fwd(const uint8_t *__restrict__ rec, int rec_bytes,
-                                                  int be, const int *__restrict__ status,
-                                                  int sstride, int ntr, int ntl,
-                                                  float dt, const float *__restrict__ tap,
-                                                  FftPlan p, float2 *__restrict__ spec,
-                                                  const float *__restrict__ fmax,
-                                                  float *__restrict__ pscale) {
-  extern __shared__ float2 sm[];
-  float2 *b0 = sm, *b1 = sm + p.m, *twm = sm + 2 * p.m, *twn = sm + 3 * p.m;
-  __shared__ float s_part[8];
-  for (int i = threadIdx.x; i < p.m; i += blockDim.x) twm[i] = p.tw_m[i];
-  for (int i = threadIdx.x; i <= p.m; i += blockDim.x) twn[i] = p.tw_n[i];
-  for (int itr = blockIdx.x; itr < ntr; itr += gridDim.x) {
-    if (status[(size_t)itr * sstride] != kAccepted) continue;  // uniform in the CTA
-    const uint8_t *r = rec + (size_t)itr * rec_bytes;
-    float *bf = reinterpret_cast<float *>(b0);
-    for (int j = threadIdx.x; j < p.n; j += blockDim.x) {
-      float v = 0.0f;
-      if (j < ntl) {
-        v = su_sample(r, j, be);
-        const float t = __fmul_rn((float)j, dt);
-        v = ((double)t < 0.1) ? __double2float_rn(__dmul_rn((double)v, 0.1 * 0.1))
-                              : __fmul_rn(v, __fmul_rn(t, t));
-        v = phys_tapered(v, j, ntl, tap);
-      }
-      bf[j] = v;
-    }
-    __syncthreads();
-    const int cur = fft_complex_smem(b0, b1, p, twm, false);
-    const float2 *Z = cur ? b1 : b0;
-    float2 *o = spec + (size_t)itr * (p.m + 1);
-    float bound = 0.0f;
-    for (int k = threadIdx.x; k <= p.m; k += blockDim.x) {
-      const float2 v = rfft_bin(Z, twn, p.m, k);
-      o[k] = v;
-      if (pscale) bound = fmaf(sqrtf(v.x * v.x + v.y * v.y), fmax[k], bound);
-    }
+template <bool PAD>
+__global__ void __launch_bounds__(kFftMaxThreads, 2)
+    k_phys_fwd(const uint8_t *__restrict__ rec, int rec_bytes, int be,
+               const int *__restrict__ status, int sstride, int ntr, int ntl, float dt,
+               const float *__restrict__ tap, const __grid_constant__ FftPlan p,
+               float2 *__restrict__ spec, const float *__restrict__ fmax,
+               float *__restrict__ pscale) {
+  extern __shared__ float4 pbuf[];
+  __shared__ float s_part[2][kFftMaxThreads / 32];
+  const int ia = 2 * blockIdx.x, ib = min(ia + 1, ntr - 1);
+  const bool oka = status[(size_t)ia * sstride] == kAccepted;
+  const bool okb = ib != ia && status[(size_t)ib * sstride] == kAccepted;
+  if (!oka && !okb) return;  // uniform in the CTA
+  const uint8_t *ra = rec + (size_t)ia * rec_bytes, *rb = rec + (size_t)ib * rec_bytes;
+  for (int j = threadIdx.x; j < p.m; j += blockDim.x) {
+    float4 v;
+    v.x = phys_sample(ra, 2 * j, be, ntl, dt, tap);
+    v.y = phys_sample(rb, 2 * j, be, ntl, dt, tap);
+    v.z = phys_sample(ra, 2 * j + 1, be, ntl, dt, tap);
+    v.w = phys_sample(rb, 2 * j + 1, be, ntl, dt, tap);
+    pbuf[stock_slot<PAD>(j)] = v;
+  }
+  __syncthreads();
+  const float4 *Z = stock_passes<false, PAD>(pbuf, pbuf, p, 0, p.nstock);
+  float2 *oa = spec + (size_t)ia * (p.m + 1), *ob = spec + (size_t)ib * (p.m + 1);
+  float ba = 0.0f, bb = 0.0f;
+  auto put = [&](int k, C2 v) {
+    const float2 re = f2_unpack(v.re), im = f2_unpack(v.im);
+    if (oka) oa[k] = make_float2(re.x, im.x);
+    if (okb) ob[k] = make_float2(re.y, im.y);
     if (pscale) {
-      for (int off = 16; off > 0; off >>= 1) bound += __shfl_xor_sync(0xffffffffu, bound, off);
-      if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = bound;
+      const float f = fmax[k];
+      ba = fmaf(sqrtf(re.x * re.x + im.x * im.x), f, ba);
+      bb = fmaf(sqrtf(re.y * re.y + im.y * im.y), f, bb);
     }
-    __syncthreads();  // Z and s_part complete; b0 / b1 free for the next trace
-    if (pscale && threadIdx.x == 0) {
-      float b = 0.0f;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) b += s_part[w];
-      b *= 2.0f;
-      int e = 0;
-      if (b > 0.0f && isfinite(b)) {
-        frexpf(b, &e);  // b = m 2^e, m in [0.5, 1)
-        e = min(max(e - 14, -126), 127);
-      }
-      pscale[itr] = ldexpf(1.0f, e);
+  };
+  for (int k = threadIdx.x; 2 * k <= p.m; k += blockDim.x) {
+    const int k2 = p.m - k;
+    C2 u, v;
+    pfa_rfft_bins(pfa_ld(Z, stock_slot<PAD>(k)), pfa_ld(Z, stock_slot<PAD>(k ? k2 : 0)),
+                  __ldg(p.tw_n + k), u, v);
+    put(k, u);
+    if (k2 != k) put(k2, v);
+  }
+  if (!pscale) return;
+  for (int off = 16; off > 0; off >>= 1) {
+    ba += __shfl_xor_sync(0xffffffffu, ba, off);
+    bb += __shfl_xor_sync(0xffffffffu, bb, off);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    s_part[0][threadIdx.x >> 5] = ba;
+    s_part[1][threadIdx.x >> 5] = bb;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 && (threadIdx.x ? okb : oka)) {
+    float b = 0.0f;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) b += s_part[threadIdx.x][w];
+    b *= 2.0f;
+    int e = 0;
+    if (b > 0.0f && isfinite(b)) {
+      frexpf(b, &e);  // b = m 2^e, m in [0.5, 1)
+      e = min(max(e - 14, -126), 127);
     }
+    pscale[threadIdx.x ? ib : ia] = ldexpf(1.0f, e);
   }
 }
 
-template <typename T>
-__device__ __forceinline__ void store_sample(T *dst, float v);
-template <>
-__device__ __forceinline__ void store_sample<float>(float *d, float v) { *d = v; }
-template <>
-__device__ __forceinline__ void store_sample<__nv_bfloat16>(__nv_bfloat16 *d, float v) {
-  *d = __float2bfloat16_rn(v);
+// Two neighbouring samples of a panel row (rows have even lengths).
+__device__ __forceinline__ void store_two(float *d, float a, float b) {
+  *reinterpret_cast<float2 *>(d) = make_float2(a, b);
 }
-template <>
-__device__ __forceinline__ void store_sample<__half>(__half *d, float v) { *d = __float2half_rn(v); }
-
-// Four output samples (two complex points) of a panel row.
-template <typename T>
-__device__ __forceinline__ void store_quad(T *dst, float mul, float2 z0, float2 z1);
-template <>
-__device__ __forceinline__ void store_quad<float>(float *d, float mul, float2 z0, float2 z1) {
-  *reinterpret_cast<float4 *>(d) = make_float4(mul * z0.x, mul * z0.y, mul * z1.x, mul * z1.y);
+__device__ __forceinline__ void store_two(__half *d, float a, float b) {
+  *reinterpret_cast<__half2 *>(d) = __floats2half2_rn(a, b);
 }
-template <>
-__device__ __forceinline__ void store_quad<__half>(__half *d, float mul, float2 z0, float2 z1) {
-  const __half2 a = __halves2half2(__float2half_rn(mul * z0.x), __float2half_rn(mul * z0.y));
-  const __half2 c = __halves2half2(__float2half_rn(mul * z1.x), __float2half_rn(mul * z1.y));
-  uint2 u;
-  u.x = *reinterpret_cast<const unsigned *>(&a);
-  u.y = *reinterpret_cast<const unsigned *>(&c);
-  *reinterpret_cast<uint2 *>(d) = u;
-}
-template <>
-__device__ __forceinline__ void store_quad<__nv_bfloat16>(__nv_bfloat16 *d, float mul, float2 z0,
-                                                         float2 z1) {
-  const __nv_bfloat162 a =
-      __halves2bfloat162(__float2bfloat16_rn(mul * z0.x), __float2bfloat16_rn(mul * z0.y));
-  const __nv_bfloat162 c =
-      __halves2bfloat162(__float2bfloat16_rn(mul * z1.x), __float2bfloat16_rn(mul * z1.y));
-  uint2 u;
-  u.x = *reinterpret_cast<const unsigned *>(&a);
-  u.y = *reinterpret_cast<const unsigned *>(&c);
-  *reinterpret_cast<uint2 *>(d) = u;
-}
-
-// Z[k] of the c2r split from a = Y[k], c = Y[m-k] (irfft_pre with the two
-// spectrum values already at hand).
-__device__ __forceinline__ float2 irfft_split(float2 a, float2 c, float2 tw) {
-  const float2 bb = cconj(c);
-  const float2 e = make_float2(0.5f * (a.x + bb.x), 0.5f * (a.y + bb.y));
-  const float2 d = make_float2(0.5f * (a.x - bb.x), 0.5f * (a.y - bb.y));
-  const float2 o = cmul(d, cconj(tw));
-  return make_float2(e.x - o.y, e.y + o.x);
+__device__ __forceinline__ void store_two(__nv_bfloat16 *d, float a, float b) {
+  *reinterpret_cast<__nv_bfloat162 *>(d) = __floats2bfloat162_rn(a, b);
 }
 
 // t*-binned panels: for every accepted trace and bin b, the filtered,
-// zero-padded spectrum X F_b -> c2r of length nffti.  A persistent CTA loads
-// the twiddles into shared memory once, then takes every gridDim.x-th trace,
-// keeps its spectrum in shared memory and runs all bins of it back to back.
-// Shared memory: two FFT buffers, the m + (m+1) twiddles, the nk-point
-// spectrum.  Each bin's input goes to the buffer the previous bin's result
-// is not in, so one barrier per bin covers the previous bin's stores.
-// Rows are stored two complex points (16 / 8 bytes) at a time when m is even.
-template <typename T>
-__global__ void __launch_bounds__(256, 3) k_phys_panels(const int *__restrict__ status, int sstride,
-                                                     int ntr, const float2 *__restrict__ spec,
-                                                     int nk, const float2 *__restrict__ filt,
-                                                     FftPlan p, int nbins, T *__restrict__ panels,
-                                                     const float *__restrict__ pscale) {
-  extern __shared__ float2 sm[];
-  float2 *twm = sm + 2 * p.m, *twn = sm + 3 * p.m, *Xs = sm + 4 * p.m + 1;
-  for (int i = threadIdx.x; i < p.m; i += blockDim.x) twm[i] = p.tw_m[i];
-  for (int i = threadIdx.x; i <= p.m; i += blockDim.x) twn[i] = p.tw_n[i];
-  int in = 0;  // buffer the next bin's input goes to
-  for (int itr = blockIdx.x; itr < ntr; itr += gridDim.x) {
+// zero-padded spectrum X F_b -> c2r of length nffti.  Two bins share every
+// instruction of the inverse transform (fft.cuh); kmax is the first frequency
+// bin past the band, where every F_b is zero.  A CTA takes (trace, group of
+// bin pairs) items, keeps the band of the trace's spectrum in shared memory
+// and runs its pairs back to back.  The first group of passes computes its
+// own inputs, a butterfly and its mirror image together (one filtered pair
+// Y[k], Y[m-k] gives both Z[k] and Z[m-k] of the c2r split), and the last
+// radix stores its outputs to the panel (neighbouring butterflies have
+// neighbouring outputs): a point crosses shared memory six times for
+// m = 3003 = 3 x 7 x 11 x 13, not ten.  With one bin per instruction, the roots
+// and twiddles in shared memory: 8.97 ms with the forward transforms for 24,902
+// traces of m = 2520, 6.37 ms for 30,000 of m = 3003, 4.80 ms for 18,432 of
+// m = 2002; now 5.2, 4.0 and 3.8 ms.  Two CTAs an SM (two 48 KB buffers each,
+// 96 registers a thread) leave it waiting for twiddles and barriers: issue
+// active 44 %.  The passes round like those of a
+// scalar transform in the same order, so a panel's half-precision values do
+// not depend on how the transform is packed or grouped.
+template <bool PAD, typename T>
+__global__ void __launch_bounds__(kFftMaxThreads, 2)
+    k_phys_panels(const int *__restrict__ status, int sstride, int ntr,
+                  const float2 *__restrict__ spec, int nk, int kmax,
+                  const float4 *__restrict__ filt, const __grid_constant__ FftPlan p, int nbins,
+                  int ngroups, T *__restrict__ panels, const float *__restrict__ pscale) {
+  extern __shared__ float4 pbuf[];
+  const int m = p.m;
+  float2 *Xs = reinterpret_cast<float2 *>(pbuf + 2 * p.swords);
+  const int npairs = (nbins + 1) / 2, per = (npairs + ngroups - 1) / ngroups;
+  // fused first group and last radix: up to 8 points a butterfly, and two
+  // groups at least
+  const int code0 = p.nstock > 1 ? p.stock[0] : 0, code1 = p.nstock > 1 ? p.stock[p.nstock - 1] : 0;
+  const bool fuse_in = p.nstock > 1 && (code0 & 15) * (code0 >> 4) <= 8;
+  const bool fuse_out = p.nstock > 1 && code1 >> 4 == 1;
+  for (int item = blockIdx.x; item < ntr * ngroups; item += gridDim.x) {
+    const int itr = item / ngroups, bp0 = (item - itr * ngroups) * per;
     if (status[(size_t)itr * sstride] != kAccepted) continue;  // uniform in the CTA
     const float2 *X = spec + (size_t)itr * nk;
-    for (int k = threadIdx.x; k < nk; k += blockDim.x) Xs[k] = X[k];
+    for (int k = threadIdx.x; k < kmax; k += blockDim.x) Xs[k] = X[k];
     __syncthreads();
     // 2 / 2^e for FP16 (exact), 2 otherwise
     const float mul = std::is_same<T, __half>::value ? 2.0f / pscale[itr] : 2.0f;
-    for (int b = 0; b < nbins; ++b) {
-      const float2 *F = filt + (size_t)b * nk;
-      float2 *b0 = sm + in * p.m, *b1 = sm + (in ^ 1) * p.m;
-      for (int k = threadIdx.x; 2 * k <= p.m; k += blockDim.x) {
-        // Y[k] and Y[m-k] of the zero-padded filtered spectrum give both
-        // Z[k] and Z[m-k] of the c2r split
-        const int k2 = p.m - k;
-        const float2 a = k < nk ? cmul(Xs[k], __ldg(F + k)) : make_float2(0.f, 0.f);
-        const float2 c = k2 < nk ? cmul(Xs[k2], __ldg(F + k2)) : make_float2(0.f, 0.f);
-        b0[k] = irfft_split(a, c, twn[k]);
-        if (k > 0 && k < k2) b0[k2] = irfft_split(c, a, twn[k2]);
-      }
-      __syncthreads();
-      const int cur = fft_complex_smem(b0, b1, p, twm, true);
-      const float2 *z = cur ? b1 : b0;
-      T *out = panels + ((size_t)itr * nbins + b) * p.n;
-      if ((p.m & 1) == 0) {  // rows of 4m bytes (FP16) / 8m bytes: 8- / 16-byte aligned
-        for (int j = threadIdx.x; 2 * j < p.m; j += blockDim.x)
-          store_quad<T>(out + 4 * j, mul, z[2 * j], z[2 * j + 1]);
+    for (int bp = bp0; bp < min(bp0 + per, npairs); ++bp) {
+      const float4 *F = filt + (size_t)bp * kmax;
+      // filtered bin k of both, zero past the band
+      auto bin = [&](int k) {
+        C2 y{0ull, 0ull};
+        if (k < kmax) {
+          const float2 x = Xs[k];
+          const float4 f = __ldg(F + k);
+          const f2 fr = f2_pack(f.x, f.y), fi = f2_pack(f.z, f.w);
+          y.re = f2_fma(f2_dup(x.x), fr, f2_mul(f2_dup(-x.y), fi));
+          y.im = f2_fma(f2_dup(x.x), fi, f2_mul(f2_dup(x.y), fr));
+        }
+        return y;
+      };
+      float4 *in = pbuf;
+      if (fuse_in) {
+        stock_by_code(code0, [&](auto cA, auto cB) {
+          constexpr int PA = decltype(cA)::value, PB = decltype(cB)::value, Q = PA * PB;
+          if constexpr (Q <= 8) {
+            const int M = m / Q;
+            auto put = [&](int n, C2 o) { pfa_st(pbuf, stock_slot<PAD>(n), o); };
+            for (int J = threadIdx.x; 2 * J <= M; J += blockDim.x) {
+              C2 u[Q], v[Q];
+#pragma unroll
+              for (int i = 0; i < Q; ++i) {
+                const int k = J + i * M;
+                pfa_irfft_pre(bin(k), bin(m - k), __ldg(p.tw_n + k), u[i], v[Q - 1 - i]);
+              }
+              stock_group<PA, PB, true>(u, J, m, 1, 0u, p.tw_m, put);
+              // butterfly 0 mirrors itself, as does the middle one
+              if (J > 0 && 2 * J < M) stock_group<PA, PB, true>(v, M - J, m, 1, 0u, p.tw_m, put);
+            }
+          }
+        });
       } else {
-        for (int j = threadIdx.x; j < p.m; j += blockDim.x) {
-          store_sample<T>(out + 2 * j, mul * z[j].x);
-          store_sample<T>(out + 2 * j + 1, mul * z[j].y);
+        for (int k = threadIdx.x; 2 * k <= m; k += blockDim.x) {
+          const int k2 = m - k;
+          C2 u, v;
+          pfa_irfft_pre(bin(k), bin(k2), __ldg(p.tw_n + k), u, v);
+          pfa_st(pbuf, stock_slot<PAD>(k), u);
+          if (k > 0 && k < k2) pfa_st(pbuf, stock_slot<PAD>(k2), v);
         }
       }
-      in = cur ? in : in ^ 1;
+      __syncthreads();
+      in = stock_passes<true, PAD>(pbuf, in, p, fuse_in ? 1 : 0, p.nstock - (fuse_out ? 1 : 0));
+      T *out = panels + ((size_t)itr * nbins + 2 * bp) * p.n;
+      const bool two = 2 * bp + 1 < nbins;
+      auto store = [&](int n, C2 z) {
+        const float2 re = f2_unpack(z.re), im = f2_unpack(z.im);
+        store_two(out + 2 * n, mul * re.x, mul * im.x);
+        if (two) store_two(out + p.n + 2 * n, mul * re.y, mul * im.y);
+      };
+      if (fuse_out) {
+        stock_by_code(code1, [&](auto cA, auto cB) {
+          constexpr int PA = decltype(cA)::value;
+          if constexpr (decltype(cB)::value == 1)
+            stock_pass<PA, 1, true, PAD>(in, m, m / PA, p.tw_m, store);
+        });
+      } else {
+        for (int j = threadIdx.x; j < m; j += blockDim.x) store(j, pfa_ld(in, stock_slot<PAD>(j)));
+      }
+      __syncthreads();  // the next pair writes pbuf (and the next item Xs)
     }
-    // the last bin's stores read the buffer other than `in`; the next trace
-    // writes Xs (read by this trace's bins, all past a barrier), then `in`
   }
 }
 
@@ -743,42 +785,6 @@ __device__ __forceinline__ bool grid_pos(float px, float py, float xc, float rdx
   fx = __fmaf_rn(__fsub_rn(px, xc), rdx, hx);
   fy = __fmaf_rn(py, rdy, hy);
   return fx >= 0.0f && fx <= (float)(nxs - 1) && fy >= 0.0f && fy <= (float)(nys - 1);
-}
-
-// Packed FP32 pairs (sm_100's f32x2 instructions): two values in one 64-bit
-// register pair, one instruction for both.  Each operation is the IEEE
-// single-precision operation of each half (round to nearest), the same
-// result as two scalar ones.
-__device__ __forceinline__ unsigned long long f2_pack(float a, float b) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float2 f2_unpack(unsigned long long r) {
-  float2 v;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(r));
-  return v;
-}
-__device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long f2_sub(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b,
-                                                     unsigned long long c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
 }
 
 // a + w (b - a) as one fused multiply-add (the form every table and sample
@@ -1704,14 +1710,6 @@ __device__ __forceinline__ void bilin_tq(const float4 *__restrict__ p, int sx, i
   v[0] = f2_lerp(f2_lerp(v00.x, v01.x, wx), f2_lerp(v10.x, v11.x, wx), wy);
   v[1] = f2_lerp(f2_lerp(v00.y, v01.y, wx), f2_lerp(v10.y, v11.y, wx), wy);
 }
-__device__ __forceinline__ unsigned long long f2_dup(float a) { return f2_pack(a, a); }
-// a + b rounded towards zero, both halves.
-__device__ __forceinline__ unsigned long long f2_add_rz(unsigned long long a,
-                                                        unsigned long long b) {
-  unsigned long long r;
-  asm("add.rz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 __device__ __forceinline__ float rsqrt_fast(float x) {
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -2559,6 +2557,29 @@ __global__ void k_any_line(const int *__restrict__ ints, size_t ints_ls, int nli
   any[i] = a ? kAccepted : 0;
 }
 
+template <typename T>
+static int launch_panels(PhysicsState *s, const FftPlan &pi, const int *status, int sstride,
+                         int ntr, int nk, const float *pscale, cudaStream_t st) {
+  auto kern = pi.spad ? k_phys_panels<true, T> : k_phys_panels<false, T>;
+  const size_t sm = 2 * sizeof(float4) * (size_t)pi.swords + sizeof(float2) * (size_t)s->kmax;
+  int rc = fft_set_smem_attr((const void *)kern, sm);
+  if (rc) return rc;
+  int dev = 0, nsm = 0, per_sm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, pi.sthreads, sm);
+  // as many CTAs as fit; a trace is split into groups of bin pairs until there
+  // are eight items per CTA (a group reloads the trace's band, 7 KB)
+  const int slots = std::max(per_sm, 1) * std::max(nsm, 1), npairs = (s->nbins + 1) / 2;
+  int ngroups = 1;
+  while (ngroups < npairs && (int64_t)ntr * ngroups < 8ll * slots) ngroups *= 2;
+  ngroups = std::min(ngroups, npairs);
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)ntr * ngroups, slots));
+  kern<<<grid, pi.sthreads, sm, st>>>(status, sstride, ntr, s->d_spec, nk, s->kmax, s->d_filter, pi,
+                              s->nbins, ngroups, (T *)s->d_panels, pscale);
+  return QPSDM_OK;
+}
+
 // Forward spectra and t*-binned panels of the traces whose status is kAccepted.
 static int run_panels(PhysicsState *s, const qpsdm_static_params &p, const PhysicsBatch &b,
                       const int *status, int sstride, cudaStream_t st, std::string *err) {
@@ -2568,49 +2589,21 @@ static int run_panels(PhysicsState *s, const qpsdm_static_params &p, const Physi
   rc = fft_plan(p.nffti, &pi, err);
   if (rc) return rc;
   const int ntr = b.ntr;
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  // persistent grids: as many CTAs as fit on the GPU, at most one per trace
-  auto grid_of = [&](const void *kern, size_t smem) {
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem);
-    return std::max(1, std::min(ntr, std::max(per_sm, 1) * std::max(nsm, 1)));
-  };
-  size_t sm = fft_smem_bytes(pf.m);
-  if ((rc = fft_set_smem_attr((const void *)k_phys_fwd, sm))) return rc;
   const bool fp16 = s->dtype == QPSDM_PANEL_FP16;
-  k_phys_fwd<<<grid_of((const void *)k_phys_fwd, sm), 256, sm, st>>>(
-      b.d_rec, b.rec_bytes, b.big_endian, status, sstride, ntr, p.ntl, p.dt, b.d_taper200, pf,
-      s->d_spec, s->d_fmax, fp16 ? s->d_pscale : nullptr);
+  const size_t sm = 2 * sizeof(float4) * (size_t)pf.swords;
+  auto fwd = pf.spad ? k_phys_fwd<true> : k_phys_fwd<false>;
+  if ((rc = fft_set_smem_attr((const void *)fwd, sm))) return rc;
+  fwd<<<(ntr + 1) / 2, pf.sthreads, sm, st>>>(b.d_rec, b.rec_bytes, b.big_endian, status, sstride,
+                                              ntr, p.ntl, p.dt, b.d_taper200, pf, s->d_spec,
+                                              s->d_fmax, fp16 ? s->d_pscale : nullptr);
   const int nk = p.nfft / 2 + 1;
-  sm = fft_smem_bytes(pi.m) + sizeof(float2) * (size_t)nk;
-  switch (s->dtype) {
-    case QPSDM_PANEL_FP32: {
-      const void *k = (const void *)k_phys_panels<float>;
-      if ((rc = fft_set_smem_attr(k, sm))) return rc;
-      k_phys_panels<float><<<grid_of(k, sm), 256, sm, st>>>(
-          status, sstride, ntr, s->d_spec, nk, s->d_filter, pi, s->nbins,
-          (float *)s->d_panels, nullptr);
-      break;
-    }
-    case QPSDM_PANEL_BF16: {
-      const void *k = (const void *)k_phys_panels<__nv_bfloat16>;
-      if ((rc = fft_set_smem_attr(k, sm))) return rc;
-      k_phys_panels<__nv_bfloat16><<<grid_of(k, sm), 256, sm, st>>>(
-          status, sstride, ntr, s->d_spec, nk, s->d_filter, pi, s->nbins,
-          (__nv_bfloat16 *)s->d_panels, nullptr);
-      break;
-    }
-    default: {
-      const void *k = (const void *)k_phys_panels<__half>;
-      if ((rc = fft_set_smem_attr(k, sm))) return rc;
-      k_phys_panels<__half><<<grid_of(k, sm), 256, sm, st>>>(
-          status, sstride, ntr, s->d_spec, nk, s->d_filter, pi, s->nbins,
-          (__half *)s->d_panels, s->d_pscale);
-    }
-  }
-  return cudaGetLastError() == cudaSuccess ? QPSDM_OK : QPSDM_ECUDA;
+  if (s->dtype == QPSDM_PANEL_FP32)
+    rc = launch_panels<float>(s, pi, status, sstride, ntr, nk, nullptr, st);
+  else if (s->dtype == QPSDM_PANEL_BF16)
+    rc = launch_panels<__nv_bfloat16>(s, pi, status, sstride, ntr, nk, nullptr, st);
+  else
+    rc = launch_panels<__half>(s, pi, status, sstride, ntr, nk, s->d_pscale, st);
+  return rc ? rc : cudaGetLastError() == cudaSuccess ? QPSDM_OK : QPSDM_ECUDA;
 }
 
 static PhysImageArgs image_args(const PhysicsState *s, const qpsdm_static_params &p,
