@@ -13,6 +13,8 @@
 #include "common.cuh"
 #include "fft.cuh"
 #include "internal.h"
+#include "ordered.cuh"
+#include "tile.cuh"
 
 namespace qpsdm {
 
@@ -212,103 +214,165 @@ int launch_spectra(const uint8_t *d_rec, int rec_bytes, int ntr, int be,
 }
 
 // ---------------------------------------------------------------------------
-// Stub imaging: one thread per image point, traces in submission order.
+// Stub imaging: traces in submission order at every point (ordered.cuh).
+//
+// Bound by issued instructions (IEEE square roots, divisions, one double
+// reciprocal per imaged pair).  9,216 traces into a 512 x 400 line (1.1e9
+// point-traces): 10.0 ms with 11 divisions and a double one for every pair;
+// 3.35 ms with the tile's dip bound, the tangents' divisions only inside the
+// taper zones, one reciprocal for the six divisions by the receiver distance
+// and the source terms kept from trace to trace.  1,024 traces into a
+// 128 x 100 line: 0.97 ms on 64 blocks, 0.13 ms with eight warps per column.
 // ---------------------------------------------------------------------------
-constexpr int kCompatBz = 32, kCompatBx = 8, kCompatChunk = 256;
 
-__global__ void __launch_bounds__(kCompatBz *kCompatBx)
+// a / b, correctly rounded, for b with the correctly rounded reciprocal y and
+// a, b in range: a quotient approximation refined twice by its exact residual
+// (P. Markstein, "Computation of elementary functions on the IBM RISC System
+// /6000 processor", IBM J. Res. Dev. 34, 1990, theorems 6 and 8: the first
+// step is within one ulp, the second rounds correctly).  One reciprocal serves
+// every division by the same distance.  In range: b in [2^-20, 2^21], a zero
+// or |a| in [2^-102, 2^104], so that no residual or quotient leaves the
+// representable numbers.
+__device__ __forceinline__ float div_by(float a, float b, float y) {
+  float q = __fmul_rn(a, y);
+  q = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+  return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+}
+// 1 / r in double, correctly rounded, for a float r in [2^-100, 2^100]: Newton
+// steps from the float reciprocal (relative error 2^-24, 2^-47, then below
+// 2^-90 before the last rounding; 1 / r has a 24-bit divisor, so it is at
+// least 2^-79 away from a rounding boundary).
+__device__ __forceinline__ double drcp_float(float r) {
+  const double d = (double)r, y0 = (double)__frcp_rn(r);
+  const double y1 = __fma_rn(y0, __fma_rn(-d, y0, 1.0), y0);
+  return __fma_rn(y1, __fma_rn(-d, y1, 1.0), y1);
+}
+// coordinates whose differences are zero or at least 2^-64
+__device__ __forceinline__ bool in_range(float v) {
+  const float a = fabsf(v);
+  return a == 0.0f || (a >= 9.094947e-13f && a <= 1.0995116e12f);  // [2^-40, 2^40]
+}
+// distances whose ratio's third power div_by reaches: [2^-20, 2^21]
+__device__ __forceinline__ bool dist_in_range(float v) {
+  return v >= 9.5367432e-7f && v <= 2097152.0f;
+}
+
+template <int SPLIT>
+__global__ void __launch_bounds__(256)
     k_image_compat(float *__restrict__ img, CompatImageArgs a,
                    const float *__restrict__ dips, const int *__restrict__ ints,
                    const float *__restrict__ geom, int ntr,
                    unsigned long long *npt) {
-  __shared__ float4 s_geom[kCompatChunk];
-  __shared__ int4 s_rng[kCompatChunk];  // ixi1, ixi2, izimin, accepted
+  constexpr int TX = 8 / SPLIT;
+  __shared__ OrderedSmem<SPLIT> sm;
+  __shared__ float s_red[8][8];
+  __shared__ TileBox s_box;
   __shared__ unsigned long long s_cnt;
-  const int tid = threadIdx.y * kCompatBz + threadIdx.x;
-  const int izi = blockIdx.x * kCompatBz + threadIdx.x;
-  const int ixb = blockIdx.y * kCompatBx + threadIdx.y;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int iz0 = blockIdx.x * 32, ixb0 = blockIdx.y * TX;
+  const int izi = iz0 + lane, ixb = ixb0 + warp / SPLIT;
   const bool live = izi < a.nzi && ixb < a.nxb;
   const int ixi = ixb + a.ixstart;
+  const bool act = live && ixi >= a.tcdp1 && ixi <= a.tcdp2;
   if (tid == 0) s_cnt = 0;
 
-  float tanx1 = 0.f, tanx2 = 0.f, tany1 = 0.f, tany2 = 0.f;
+  float tan[4] = {0.f, 0.f, 0.f, 0.f};
   float acc = 0.0f;
-  const bool in_table = ixi >= a.tcdp1 && ixi <= a.tcdp2;
   if (live) {
     const size_t k = (size_t)ixi * a.nzi + izi;
-    tanx1 = dips[k];
-    tanx2 = dips[a.nxz + k];
-    tany1 = dips[2 * a.nxz + k];
-    tany2 = dips[3 * a.nxz + k];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) tan[j] = dips[j * a.nxz + k];
     acc = img[(size_t)ixb * a.nzi + izi];
   }
   // Per-point constants of image_depth_gpu (src/q-psdm.cu:2303-2330).
   const float tz = a.taperzone;
-  const float tanx1c = __fsub_rn(tanx1, __fmul_rn(tz, __fadd_rn(1.0f, __fmul_rn(tanx1, tanx1))));
-  const float tanx2c = __fadd_rn(tanx2, __fmul_rn(tz, __fadd_rn(1.0f, __fmul_rn(tanx2, tanx2))));
-  const float tany1c = __fsub_rn(tany1, __fmul_rn(tz, __fadd_rn(1.0f, __fmul_rn(tany1, tany1))));
-  const float tany2c = __fadd_rn(tany2, __fmul_rn(tz, __fadd_rn(1.0f, __fmul_rn(tany2, tany2))));
+  DipLimits d;
+  d.x1 = tan[0], d.x2 = tan[1], d.y1 = tan[2], d.y2 = tan[3];
+  d.x1c = __fsub_rn(d.x1, __fmul_rn(tz, __fadd_rn(1.0f, __fmul_rn(d.x1, d.x1))));
+  d.x2c = __fadd_rn(d.x2, __fmul_rn(tz, __fadd_rn(1.0f, __fmul_rn(d.x2, d.x2))));
+  d.y1c = __fsub_rn(d.y1, __fmul_rn(tz, __fadd_rn(1.0f, __fmul_rn(d.y1, d.y1))));
+  d.y2c = __fadd_rn(d.y2, __fmul_rn(tz, __fadd_rn(1.0f, __fmul_rn(d.y2, d.y2))));
+  d.wide = d.x1 > d.x1c && d.x2 < d.x2c && d.y1 > d.y1c && d.y2 < d.y2c;
   const float z = __fmul_rn((float)izi, a.dzi);
   const float z2 = __fmul_rn(z, z);
   const float x = __fmul_rn((float)ixi, a.dxi);
+  tile_limits(act, d.x1c, d.x2c, d.y1c, d.y2c, s_red);
+  // the tile's columns inside the tables, and its rows
+  const int col_lo = max(ixb0 + a.ixstart, a.tcdp1);
+  const int col_hi = min(min(ixb0 + TX, a.nxb) - 1 + a.ixstart, a.tcdp2);
+  const int nrow = min(32, a.nzi - iz0);
+  __syncthreads();
+  if (tid == 0)
+    s_box = tile_box(s_red, col_lo * a.dxi, col_hi * a.dxi, iz0 * a.dzi,
+                     (iz0 + nrow - 1) * a.dzi);
   // ts = tg = 1 in the reference: t, the sample indices and v are constants.
-  const float ts = 1.0f, tg = 1.0f;
-  const float t = __fadd_rn(ts, tg);
+  const float t = 2.0f;
   const int it1 = __float2int_rz(__fdiv_rn(t, a.dt1));
   const bool t_ok = it1 > 0 && it1 + 1 < a.nt;
   const float v0 = ((double)t > 0.1) ? __fdiv_rn(100.0f, __fmul_rn(t, t))
                                      : __fmul_rn(100.0f, 100.0f);
+  const bool z_ok = in_range(z) && in_range(x);
   unsigned cnt = 0;
+  // source terms, reused while consecutive traces share a source
+  float last_sx = NAN, last_sy = NAN, ds = 0.f, sax = 0.f, say = 0.f, saz = 0.f;
 
-  for (int c0 = 0; c0 < ntr; c0 += kCompatChunk) {
-    const int nc = min(kCompatChunk, ntr - c0);
-    __syncthreads();
-    for (int i = tid; i < nc; i += blockDim.x * blockDim.y) {
-      const int *q = ints + (size_t)(c0 + i) * kGateInts;
-      const float *gq = geom + (size_t)(c0 + i) * kGateF;
-      s_rng[i] = make_int4(q[4], q[5], q[7], q[0] == kAccepted);
-      s_geom[i] = make_float4(gq[0], gq[1], gq[2], gq[3]);
+  auto keep = [&](int i, int4 &r, float4 &g, float2 &h) {
+    h = make_float2(0.0f, 0.0f);
+    const int4 q0 = *reinterpret_cast<const int4 *>(ints + (size_t)i * kGateInts);
+    if (q0.x != kAccepted) return false;
+    const int4 q1 = *reinterpret_cast<const int4 *>(ints + (size_t)i * kGateInts + 4);
+    const int lo = max(q1.x, col_lo), hi = min(q1.y, col_hi);
+    const int rows = iz0 + nrow - max(q1.w, iz0);
+    if (lo > hi || rows <= 0) return false;
+    cnt += (unsigned)((hi - lo + 1) * rows);  // a point-trace: a pair in the aperture
+    g = *reinterpret_cast<const float4 *>(geom + (size_t)i * kGateF);
+    const bool ok = in_range(g.x) && in_range(g.y) && in_range(g.z) && in_range(g.w);
+    r = make_int4(lo, hi, q1.w, ok);
+    return t_ok && tile_keep(make_float2(g.x, g.y), make_float2(g.z, g.w), s_box);
+  };
+  auto eval = [&](int k, float &val) {
+    const int4 r = sm.rec[k];
+    const float4 gm = sm.geo[k];
+    if (ixi < r.x || ixi > r.y || izi < r.z) return false;
+    if (gm.x != last_sx || gm.y != last_sy) {
+      last_sx = gm.x;
+      last_sy = gm.y;
+      const float dsx = __fsub_rn(gm.x, x);
+      ds = __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(dsx, dsx), __fmul_rn(gm.y, gm.y)), z2));
+      sax = __fdiv_rn(dsx, ds), say = __fdiv_rn(gm.y, ds), saz = __fdiv_rn(z, ds);
     }
-    __syncthreads();
-    if (!live || !in_table) continue;
-    for (int i = 0; i < nc; ++i) {
-      const int4 rg = s_rng[i];
-      if (!rg.w || ixi < rg.x || ixi > rg.y || izi < rg.z) continue;
-      ++cnt;
-      const float4 gm = s_geom[i];
-      const float dsx = __fsub_rn(gm.x, x), dgx = __fsub_rn(gm.z, x);
-      const float ds = __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(dsx, dsx), __fmul_rn(gm.y, gm.y)), z2));
-      const float dg = __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(dgx, dgx), __fmul_rn(gm.w, gm.w)), z2));
-      const float ux = __fadd_rn(__fdiv_rn(dsx, ds), __fdiv_rn(dgx, dg));
-      const float uy = __fadd_rn(__fdiv_rn(gm.y, ds), __fdiv_rn(gm.w, dg));
-      const float uz = __fadd_rn(__fdiv_rn(z, ds), __fdiv_rn(z, dg));
-      const float tanx = __fdiv_rn(ux, uz), tany = __fdiv_rn(uy, uz);
-      // The reference rejects `tanx <= tanx1c || tanx2c <= tanx || ...`; the
-      // negated form agrees for every number and also rejects a NaN tangent
-      // (0/0 at z = 0 for collinear source, receiver and node), as the
-      // reference binary does: its approximate divisions give +-inf there.
-      if (!(tanx > tanx1c && tanx < tanx2c && tany > tany1c && tany < tany2c)) continue;
-      float w = 1.0f;
-      if (tanx < tanx1) w = __fmul_rn(w, __fdiv_rn(__fsub_rn(tanx, tanx1c), __fsub_rn(tanx1, tanx1c)));
-      if (tanx > tanx2) w = __fmul_rn(w, __fdiv_rn(__fsub_rn(tanx2c, tanx), __fsub_rn(tanx2c, tanx2)));
-      if (tany < tany1) w = __fmul_rn(w, __fdiv_rn(__fsub_rn(tany, tany1c), __fsub_rn(tany1, tany1c)));
-      if (tany > tany2) w = __fmul_rn(w, __fdiv_rn(__fsub_rn(tany2c, tany), __fsub_rn(tany2c, tany2)));
-      if (!t_ok) continue;
-      // tr = ds/dg*ds/dg*ds/dg*tg/ts, evaluated left to right.
-      float r = __fdiv_rn(ds, dg);
-      r = __fdiv_rn(__fmul_rn(r, ds), dg);
-      r = __fdiv_rn(__fmul_rn(r, ds), dg);
-      r = __fdiv_rn(__fmul_rn(r, tg), ts);
-      const double rd = (double)r;
-      r = __double2float_rn(__dmul_rn((double)w, __dadd_rn(rd, __ddiv_rn(1.0, rd))));
-      acc = __fadd_rn(acc, __fmul_rn(v0, r));
-    }
-  }
-  if (live) img[(size_t)ixb * a.nzi + izi] = acc;
+    const float dgx = __fsub_rn(gm.z, x);
+    const float dg =
+        __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(dgx, dgx), __fmul_rn(gm.w, gm.w)), z2));
+    const float y = __frcp_rn(dg);
+    // no quotient leaves div_by's range
+    const bool fast = r.w && z_ok && dist_in_range(dg) && dist_in_range(ds);
+    auto over_dg = [&](float n) { return fast ? div_by(n, dg, y) : __fdiv_rn(n, dg); };
+    const float ux = __fadd_rn(sax, over_dg(dgx));
+    const float uy = __fadd_rn(say, over_dg(gm.w));
+    const float uz = __fadd_rn(saz, over_dg(z));
+    // The reference rejects `tanx <= tanx1c || tanx2c <= tanx || ...`; the
+    // negated form agrees for every number and also rejects a NaN tangent
+    // (0/0 at z = 0 for collinear source, receiver and node), as the
+    // reference binary does: its approximate divisions give +-inf there.
+    float w;
+    if (!dip_taper(ux, uy, uz, d, w)) return false;
+    // tr = ds/dg*ds/dg*ds/dg*tg/ts, evaluated left to right (tg = ts = 1).
+    float q = over_dg(ds);
+    q = over_dg(__fmul_rn(q, ds));
+    q = over_dg(__fmul_rn(q, ds));
+    const double rd = (double)q;
+    const double ri = q >= 7.9e-31f && q <= 1.26e30f ? drcp_float(q) : __ddiv_rn(1.0, rd);
+    q = __double2float_rn(__dmul_rn((double)w, __dadd_rn(rd, ri)));
+    val = __fmul_rn(v0, q);
+    return true;
+  };
+  ordered_walk<SPLIT>(sm, ntr, act, keep, eval, [&](float v) { acc = __fadd_rn(acc, v); });
+  if (live && (SPLIT == 1 || warp % SPLIT == 0)) img[(size_t)ixb * a.nzi + izi] = acc;
   if (npt) {
     // warp-aggregate the point-trace count
     for (int off = 16; off > 0; off >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, off);
-    if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(&s_cnt, (unsigned long long)cnt);
+    if (lane == 0 && cnt) atomicAdd(&s_cnt, (unsigned long long)cnt);
     __syncthreads();
     if (tid == 0 && s_cnt) atomicAdd(npt, s_cnt);
   }
@@ -319,9 +383,11 @@ int launch_image_compat(float *d_img, const CompatImageArgs &a,
                         const float *d_geom, int ntr, unsigned long long *d_npt,
                         cudaStream_t s) {
   if (ntr <= 0) return QPSDM_OK;
-  dim3 block(kCompatBz, kCompatBx);
-  dim3 grid((a.nzi + kCompatBz - 1) / kCompatBz, (a.nxb + kCompatBx - 1) / kCompatBx);
-  k_image_compat<<<grid, block, 0, s>>>(d_img, a, d_dips, d_ints, d_geom, ntr, d_npt);
+  ordered_by_split(a.nzi, a.nxb, 32, [&](auto split) {
+    constexpr int S = decltype(split)::value;
+    const dim3 grid((a.nzi + 31) / 32, (a.nxb + 8 / S - 1) / (8 / S));
+    k_image_compat<S><<<grid, 256, 0, s>>>(d_img, a, d_dips, d_ints, d_geom, ntr, d_npt);
+  });
   return cudaGetLastError() == cudaSuccess ? QPSDM_OK : QPSDM_ECUDA;
 }
 
