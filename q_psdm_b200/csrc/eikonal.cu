@@ -150,9 +150,11 @@ __global__ void k_eik_setup(const float *__restrict__ vel, const float *__restri
 
 // One in-place Godunov relaxation of the listed blocks (sweep 0: every block).
 //
-// A sweep of all 28 M nodes of 32 sources took 0.27 ms, bound by the 64-bit
-// divisions of a flat node index, and 256 sweeps 70 ms, although a block is
-// active in about 60 of them.
+// Bound by issue (64 % active) and the loads' latency.  A sweep of all 28 M nodes
+// of 32 sources took 0.27 ms, with the 64-bit divisions of a flat node index,
+// and 256 sweeps 70 ms, although a block changes in about 60 of them: 15.4 ms
+// now.  (Listing a neighbour only where its value is the larger one took more
+// registers than it saved blocks: 23.5 ms.)
 __global__ void __launch_bounds__(kEikThreads)
     k_eik_relax(const float *__restrict__ F, float *__restrict__ T, EikBlocks B, int sweep) {
   __shared__ unsigned s_faces;
@@ -207,13 +209,15 @@ __global__ void __launch_bounds__(kEikThreads)
   }
 }
 
-// t* of the listed blocks along the upwind directions of T (FP64): a block
-// with its halo in shared memory is relaxed until nothing in it changes.  In
-// sweep 0 the blocks that hold start nodes, and after it what they reach: t*
-// at a node depends on nodes of smaller T only, so the values settle outwards
-// from the source, most blocks in a few visits.  (256 sweeps over every node
-// took 95 ms for the 28 M nodes.)
-__global__ void __launch_bounds__(kEikThreads)
+// t* of the listed blocks along the upwind directions of T (FP64), one node a
+// thread: a block with its halo in shared memory is relaxed until nothing in
+// it changes.  In sweep 0 the blocks that hold start nodes, and after it what
+// they reach: t* at a node depends on nodes of smaller T only, so the values
+// settle outwards from the source, most blocks in a few visits, and a block is
+// listed only for a changed neighbour of smaller T.  (256 sweeps over every
+// node took 95 ms for the 28 M nodes of 32 sources; 6.9 ms now.)
+constexpr int kTsThreads = kEx * kEy * kEz;
+__global__ void __launch_bounds__(kTsThreads)
     k_tstar_relax(const float *__restrict__ F, const float *__restrict__ T,
                   const float *__restrict__ QF, double *__restrict__ TS, EikBlocks B, int sweep) {
   constexpr int HX = kEx + 2, HY = kEy + 2, HZ = kEz + 2;
@@ -224,68 +228,50 @@ __global__ void __launch_bounds__(kEikThreads)
   const double ih2 = 1.0 / ((double)g.h * g.h);
   const int n = sweep == 0 ? B.nblk : (int)B.count[sweep % 3];
   if (blockIdx.x == 0 && threadIdx.x == 0) B.count[(sweep + 2) % 3] = 0;
+  const int lx = threadIdx.x % kEx, ly = threadIdx.x / kEx % kEy, lz = threadIdx.x / (kEx * kEy);
+  const int at = ((lz + 1) * HY + ly + 1) * HX + lx + 1;
   for (int k = blockIdx.x; k < n; k += gridDim.x) {
     const int blk = sweep == 0 ? k : B.list[sweep & 1][k];
     const EikBlock e = eik_block(B, blk);
-    // this thread's two nodes: where, and the update's terms
-    int at[2], nb[2][3];
-    size_t gi[2];
-    double w[2][3], q[2], rden[2], val[2], old[2];
-    bool on[2], start = false;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int l = threadIdx.x + h * kEikThreads;
-      const int lx = l % kEx, ly = l / kEx % kEy, lz = l / (kEx * kEy);
-      const int ix = e.x0 + lx, iy = e.y0 + ly, iz = e.z0 + lz;
-      at[h] = ((lz + 1) * HY + ly + 1) * HX + lx + 1;
-      gi[h] = e.base + lz * sxy + (size_t)ly * g.nx + lx;
-      on[h] = ix < g.nx && iy < g.ny && iz < g.nz;
-      w[h][0] = w[h][1] = w[h][2] = 0.0;
-      nb[h][0] = nb[h][1] = nb[h][2] = at[h];
-      q[h] = rden[h] = val[h] = old[h] = 0.0;
-      if (!on[h]) continue;
-      const size_t i = gi[h];
-      val[h] = old[h] = TS[i];
-      const bool st = F[i] < 0.0f;
-      start = start || st;
+    const int ix = e.x0 + lx, iy = e.y0 + ly, iz = e.z0 + lz;
+    const size_t i = e.base + lz * sxy + (size_t)ly * g.nx + lx;
+    // the update's terms: upwind neighbours and weights
+    int nb[3] = {at, at, at};
+    double w[3] = {0.0, 0.0, 0.0}, q = 0.0, rden = 0.0, val = 0.0, old = 0.0;
+    unsigned faces = 0;  // sides whose outside neighbour lies downwind
+    bool on = ix < g.nx && iy < g.ny && iz < g.nz, start = false;
+    if (on) {
+      val = old = TS[i];
+      start = F[i] < 0.0f;
       const float ti = T[i];
-      on[h] = !st && ti < kInf;
-      if (!on[h]) continue;
       const size_t sd[3] = {1, (size_t)g.nx, sxy};
       const int hd[3] = {1, HX, HX * HY};
       const int id[3] = {ix, iy, iz}, nd[3] = {g.nx, g.ny, g.nz};
       double den = 0.0;
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        float best = ti;
-        int o = 0;
-        if (id[d] > 0 && T[i - sd[d]] < best) {
-          best = T[i - sd[d]];
-          o = -hd[d];
+        const float lo = id[d] > 0 ? T[i - sd[d]] : kInf;
+        const float hi = id[d] < nd[d] - 1 ? T[i + sd[d]] : kInf;
+        const float best = fminf(lo, hi);
+        if (best < ti) {
+          w[d] = ((double)ti - (double)best) * ih2;
+          nb[d] = at + (lo <= hi ? -hd[d] : hd[d]);
+          den += w[d];
         }
-        if (id[d] < nd[d] - 1 && T[i + sd[d]] < best) {
-          best = T[i + sd[d]];
-          o = hd[d];
-        }
-        if (o) {
-          w[h][d] = ((double)ti - (double)best) * ih2;
-          nb[h][d] = at[h] + o;
-          den += w[h][d];
-        }
+        faces |= (lo > ti ? 2u : 0u) << (2 * d) | (hi > ti ? 4u : 0u) << (2 * d);
       }
-      q[h] = QF[i];
-      if (den > 0.0)
-        rden[h] = 1.0 / den;
-      else
-        on[h] = false;
+      faces &= eik_faces(lx, ly, lz);
+      q = QF[i];
+      on = !start && ti < kInf && den > 0.0;
+      if (on) rden = 1.0 / den;
     }
     if (threadIdx.x == 0) s_faces = 0;
     const bool seed = __syncthreads_or(start);
     if (sweep == 0 && !seed) continue;  // uniform in the CTA
-    for (int j = threadIdx.x; j < HX * HY * HZ; j += kEikThreads) {
+    for (int j = threadIdx.x; j < HX * HY * HZ; j += kTsThreads) {
       const int hx = j % HX, hy = j / HX % HY, hz = j / (HX * HY);
-      const int ix = e.x0 + hx - 1, iy = e.y0 + hy - 1, iz = e.z0 + hz - 1;
-      const bool in = ix >= 0 && ix < g.nx && iy >= 0 && iy < g.ny && iz >= 0 && iz < g.nz;
+      const int jx = e.x0 + hx - 1, jy = e.y0 + hy - 1, jz = e.z0 + hz - 1;
+      const bool in = jx >= 0 && jx < g.nx && jy >= 0 && jy < g.ny && jz >= 0 && jz < g.nz;
       s_ts[j] = in ? TS[e.base + (ptrdiff_t)(hz - 1) * (ptrdiff_t)sxy +
                         (ptrdiff_t)(hy - 1) * g.nx + (hx - 1)]
                    : 0.0;
@@ -294,33 +280,22 @@ __global__ void __launch_bounds__(kEikThreads)
     bool more = true;
     for (int it = 0; it < 64 && more; ++it) {
       bool ch = false;
+      if (on) {
+        double num = q;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (!on[h]) continue;
-        double num = q[h];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) num += w[h][d] * s_ts[nb[h][d]];
-        const double v = num * rden[h];
+        for (int d = 0; d < 3; ++d) num += w[d] * s_ts[nb[d]];
+        const double v = num * rden;
         // (bits: a NaN settles too)
-        if (__double_as_longlong(v) != __double_as_longlong(val[h])) {
-          val[h] = v;
-          s_ts[at[h]] = v;
-          ch = true;
-        }
+        ch = __double_as_longlong(v) != __double_as_longlong(val);
+        if (ch) s_ts[at] = val = v;
       }
       more = __syncthreads_or(ch);
     }
-    unsigned faces = 0;
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-      if (on[h] && __double_as_longlong(val[h]) != __double_as_longlong(old[h])) {
-        const int l = threadIdx.x + h * kEikThreads;
-        TS[gi[h]] = val[h];
-        faces |= eik_faces(l % kEx, l / kEx % kEy, l / (kEx * kEy));
-      }
-    faces &= ~1u;                     // settled, unless the loop ran out
-    if (more) faces |= 1u;
-    if (sweep == 0) faces |= 0x7eu;  // start nodes may fill the block
+    if (on && __double_as_longlong(val) != __double_as_longlong(old))
+      TS[i] = val;
+    else if (sweep > 0)
+      faces = 0;  // (start nodes may fill the block: sweep 0 lists what is downwind of them)
+    if (more) faces |= 1u;  // settled, unless the loop ran out
     if (faces) atomicOr(&s_faces, faces);
     __syncthreads();
     eik_mark(B, blk, e, s_faces, sweep);
@@ -445,7 +420,7 @@ extern "C" int qpsdm_eikonal_solve(const float *d_vel, const float *d_invq,
   cudaMemsetAsync(B.count, 0, 3 * sizeof(unsigned), st);
   cudaMemsetAsync(B.listed, 0xff, sizeof(int) * (size_t)nblk, st);
   rc = relax(4 * (g.nx + g.ny + g.nz), [&](int sweep) {
-    k_tstar_relax<<<grd, kEikThreads, 0, st>>>(F, d_T, QF, TS, B, sweep);
+    k_tstar_relax<<<grd, kTsThreads, 0, st>>>(F, d_T, QF, TS, B, sweep);
   });
   if (rc) return rc;
   k_tstar_store<<<148 * 8, 256, 0, st>>>(TS, d_tstar, n);
