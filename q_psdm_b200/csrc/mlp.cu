@@ -11,11 +11,14 @@
 // access is fixed by its warp index -- and column half (w / 4), so the
 // epilogue of a layer (bias, SiLU, BF16 store) is spread over 256 threads.
 //
-// Inference: two teams per CTA work on two tiles at once, each with its own
+// Inference: three teams per CTA work on three tiles at once, each with its own
 // mbarrier, TMEM columns and activation buffer (a layer's output overwrites
 // its input once the MMA that read it has completed), so one team's MMAs run
-// while the other team is in its epilogue.  Each thread loads its inputs of
-// the next tile while the current one is computed.
+// while the others are in their epilogues.  Each thread loads its inputs of
+// the next tile while the current one is computed.  The special-function
+// queue bounds it (512 tanh a sample, 16 a cycle per SM: 3.0 ms for 26 M
+// samples); with two teams the queue ran dry while both waited for their MMAs:
+// 5.96 ms, three teams and biases read four to a load: 4.98 ms.
 //
 // Training: one team per CTA.  Backward re-computes what it needs (all
 // activations do not fit in shared memory next to the weights) and forms
@@ -71,9 +74,10 @@ constexpr int sDb = sBias + kBiasBytes;       // fp32 bias-gradient partials [4 
 constexpr int sLoss = sDb + 4 * kH * 4;       // fp32 loss partials [8 warps]
 constexpr int kSmem = sLoss + 32;             // 214,112 bytes
 // inference shared memory map: weights, biases, then per team X and H
+constexpr int kFwdTeams = 3;
 constexpr int fBias = kWBytes;
 constexpr int fTeam0 = fBias + 2304;
-constexpr int kFwdSmem = fTeam0 + 2 * (kXBytes + kHBytes);  // 182,528 bytes
+constexpr int kFwdSmem = fTeam0 + kFwdTeams * (kXBytes + kHBytes);  // 219,392 bytes
 
 struct MlpTileArgs {
   float in_scale[5], in_shift[5];  // features = (raw - shift) * scale
@@ -183,16 +187,32 @@ __device__ __forceinline__ void acc_ld16(uint32_t acc, const Role &ro, int c0, f
   tc::tmem_ld16(acc + ro.lane_base + c0, v);
 }
 
-// H = SiLU(acc + b) for this thread's 64 columns, into a [128][128] buffer.
+// H = SiLU(acc + b) for this thread's 64 columns, into a [128][128] buffer, 32
+// columns at a time (80 registers hold three teams of 256 threads an SM).
+// The biases are read four to a load: with one each, they were half of the
+// epilogue's instructions to the shared-memory and special-function queue.
 __device__ __forceinline__ void epi_silu(uint32_t acc, const Role &ro, const float *hb,
                                          uint8_t *hout) {
-  const int c0 = ro.half * 64;
-  float v[64];
-  acc_ld64(acc, ro, c0, v);
 #pragma unroll
-  for (int i = 0; i < 64; ++i) v[i] = silu_h(fmaf(0.5f, v[i], hb[c0 + i]));
+  for (int h = 0; h < 2; ++h) {
+    const int c0 = ro.half * 64 + 32 * h;
+    uint32_t r[32];
+    tc::tmem_ld16_nowait(acc + ro.lane_base + c0, r);
+    tc::tmem_ld16_nowait(acc + ro.lane_base + c0 + 16, r + 16);
+    tc::tmem_wait_ld_dep16(r);
+    tc::tmem_wait_ld_dep16(r + 16);
+    float v[32];
 #pragma unroll
-  for (int k = 0; k < 8; ++k) st_row8(hout, ro.row, c0 + 8 * k, kH, v + 8 * k);
+    for (int i = 0; i < 8; ++i) {
+      const float4 b = *reinterpret_cast<const float4 *>(hb + c0 + 4 * i);
+      v[4 * i] = silu_h(fmaf(0.5f, __uint_as_float(r[4 * i]), b.x));
+      v[4 * i + 1] = silu_h(fmaf(0.5f, __uint_as_float(r[4 * i + 1]), b.y));
+      v[4 * i + 2] = silu_h(fmaf(0.5f, __uint_as_float(r[4 * i + 2]), b.z));
+      v[4 * i + 3] = silu_h(fmaf(0.5f, __uint_as_float(r[4 * i + 3]), b.w));
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) st_row8(hout, ro.row, c0 + 8 * k, kH, v + 8 * k);
+  }
 }
 
 // Normalised features of one sample into the X tile (zero padding to 16).
@@ -236,20 +256,19 @@ __device__ __forceinline__ void load_weights(uint8_t *sm, float *bias,
 }
 
 // ---------------------------------------------------------------------------
-// inference: y[n][2] from x[n][5]; two teams of 256 threads per CTA
+// inference: y[n][2] from x[n][5]; three teams of 256 threads per CTA
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(2 * kTeam, 1)
+__global__ void __launch_bounds__(kFwdTeams * kTeam, 1)
     k_mlp_forward(const uint8_t *__restrict__ wimg, const float *__restrict__ params,
                   const float *__restrict__ x, int nsamp, MlpTileArgs ta, float *__restrict__ y,
                   int *err) {
   extern __shared__ __align__(1024) uint8_t sm[];
-  __shared__ uint64_t bars[2];
+  __shared__ uint64_t bars[kFwdTeams];
   __shared__ uint32_t tslot;
   const int tid = threadIdx.x, team_id = tid / kTeam, t = tid % kTeam;
-  if (tid < 32) tc::tmem_alloc(&tslot, 256);
+  if (tid < 32) tc::tmem_alloc(&tslot, 512);  // 128 columns a team, a power of two
   if (tid == 0) {
-    tc::mbar_init(&bars[0], 1);
-    tc::mbar_init(&bars[1], 1);
+    for (int i = 0; i < kFwdTeams; ++i) tc::mbar_init(&bars[i], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   float *bias = reinterpret_cast<float *>(sm + fBias);
@@ -265,16 +284,17 @@ __global__ void __launch_bounds__(2 * kTeam, 1)
   // this thread's inputs of its next tile, loaded one tile ahead
   float raw[5];
   {
-    const int s0 = (2 * blockIdx.x + team_id) * kTile + ro.row;
+    const int s0 = (kFwdTeams * blockIdx.x + team_id) * kTile + ro.row;
     load_raw(x, s0, ro.half == 0 && s0 < nsamp, raw);
   }
-  for (int tile = 2 * blockIdx.x + team_id; tile < ntiles; tile += 2 * gridDim.x) {
+  for (int tile = kFwdTeams * blockIdx.x + team_id; tile < ntiles;
+       tile += kFwdTeams * gridDim.x) {
     const int s = tile * kTile + ro.row;
     const bool live = s < nsamp;
     if (ro.half == 0) {
       put_raw(sx, ro.row, raw, live, ta);
-      const int sn = s + 2 * gridDim.x * kTile;
-      load_raw(x, sn, sn < nsamp, raw);
+      const int ahead = kFwdTeams * gridDim.x * kTile;
+      load_raw(x, s + ahead, s < nsamp - ahead, raw);
     }
     if (!g.run(acc, sx, kIn, 0, sm + sW1, kIn, 0, kH, kIn)) break;
     epi_silu(acc, ro, bias, sh);
@@ -295,7 +315,7 @@ __global__ void __launch_bounds__(2 * kTeam, 1)
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (tid < 32) tc::tmem_free(tslot, 256);
+  if (tid < 32) tc::tmem_free(tslot, 512);
 }
 
 // ---------------------------------------------------------------------------
@@ -736,9 +756,9 @@ extern "C" int qpsdm_mlp_forward(qpsdm_mlp *h, const float *d_x, int n, float *d
                                  void *stream) {
   if (!h || !d_x || !d_y || n <= 0) return QPSDM_EINVAL;
   cudaSetDevice(h->device);
-  const int pairs = ((n + kTile - 1) / kTile + 1) / 2;
-  const int grid = pairs < h->nsm ? pairs : h->nsm;
-  k_mlp_forward<<<grid, 2 * kTeam, kFwdSmem, (cudaStream_t)stream>>>(h->wimg, h->p, d_x, n,
+  const int ctas = ((n + kTile - 1) / kTile + kFwdTeams - 1) / kFwdTeams;
+  const int grid = ctas < h->nsm ? ctas : h->nsm;
+  k_mlp_forward<<<grid, kFwdTeams * kTeam, kFwdSmem, (cudaStream_t)stream>>>(h->wimg, h->p, d_x, n,
                                                                      h->ta, d_y, h->err);
   return cudaGetLastError() == cudaSuccess ? QPSDM_OK : QPSDM_ECUDA;
 }
