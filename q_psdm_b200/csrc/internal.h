@@ -74,6 +74,11 @@ struct FftPlan;
 int fft_plan(int n, FftPlan *out, std::string *err);
 int fft_set_smem_attr(const void *kernel, size_t bytes);
 
+// The workspace a network handle keeps for the table calls (mlp.cu).
+void *mlp_take_workspace(qpsdm_mlp *h, size_t bytes, size_t *got);
+void mlp_put_workspace(qpsdm_mlp *h, void *p, size_t bytes);
+int mlp_device(const qpsdm_mlp *h);
+
 // Gate of a trace batch (src/q-psdm.cu:2107-2171), one thread per trace.
 struct GateArgs {
   double scaled, fxi, cyi;

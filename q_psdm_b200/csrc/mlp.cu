@@ -38,9 +38,12 @@
 #include <cuda_bf16.h>
 #include <math.h>
 
+#include <mutex>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
+#include "internal.h"
 #include "qpsdm_engine.h"
 #include "tc.cuh"
 
@@ -590,7 +593,47 @@ struct qpsdm_mlp {
   int *err = nullptr;
   int64_t step = 0;
   MlpTileArgs ta{};
+  // one workspace of the table calls (surrogate.cu), kept between them
+  std::mutex ws_mu;
+  void *ws = nullptr;
+  size_t ws_bytes = 0;
 };
+
+namespace qpsdm {
+
+// A device workspace of at least `bytes` for a call that ends with its work
+// done: the one the handle keeps if it is free and large enough, else a new
+// one.  mlp_put_workspace keeps it in the handle again (the larger of two
+// when calls overlapped) or frees it.
+void *mlp_take_workspace(qpsdm_mlp *h, size_t bytes, size_t *got) {
+  {
+    std::lock_guard<std::mutex> lk(h->ws_mu);
+    if (h->ws && h->ws_bytes >= bytes) {
+      void *p = h->ws;
+      *got = h->ws_bytes;
+      h->ws = nullptr;
+      h->ws_bytes = 0;
+      return p;
+    }
+  }
+  void *p = nullptr;
+  *got = bytes;
+  return cudaMalloc(&p, bytes) == cudaSuccess ? p : nullptr;
+}
+void mlp_put_workspace(qpsdm_mlp *h, void *p, size_t bytes) {
+  if (!p) return;
+  {
+    std::lock_guard<std::mutex> lk(h->ws_mu);
+    if (bytes > h->ws_bytes) {
+      std::swap(p, h->ws);
+      h->ws_bytes = bytes;
+    }
+  }
+  cudaFree(p);
+}
+int mlp_device(const qpsdm_mlp *h) { return h->device; }
+
+}  // namespace qpsdm
 
 static int mlp_grid(const qpsdm_mlp *h, int nsamp) {
   const int ntiles = (nsamp + kTile - 1) / kTile;
@@ -656,6 +699,7 @@ extern "C" int qpsdm_mlp_destroy(qpsdm_mlp *h) {
   cudaFree(h->slices);
   cudaFree(h->wimg);
   cudaFree(h->err);
+  cudaFree(h->ws);
   delete h;
   return QPSDM_OK;
 }
