@@ -161,19 +161,27 @@ __device__ __forceinline__ void tmem_wait_ld_dep16(uint32_t *r) {
 }
 
 // D (TMEM, 128 lanes x N columns at d_tmem) (+)= A * B^T over K (multiple of
-// 16).  A: 128 x K; B: N x K.  a_desc0/b_desc0 describe the first K = 16
-// step; each further step advances the start addresses by a_step/b_step
-// bytes.  Issued by the calling thread only; commits to *bar.
-__device__ __forceinline__ void gemm_issue(uint32_t d_tmem, uint32_t a_saddr, uint32_t a_lbo,
+// 16).  A: 128 x K; B: N x K.  a_saddr/b_saddr with their offsets describe
+// the first K = 16 step; each further step advances the start addresses by
+// a_step/b_step bytes.  Issued by the calling thread only, without a commit.
+__device__ __forceinline__ void gemm_steps(uint32_t d_tmem, uint32_t a_saddr, uint32_t a_lbo,
                                            uint32_t a_sbo, uint32_t a_step, uint32_t b_saddr,
                                            uint32_t b_lbo, uint32_t b_sbo, uint32_t b_step,
-                                           uint32_t idesc, int K, bool accumulate,
-                                           uint64_t *bar) {
+                                           uint32_t idesc, int K, bool accumulate) {
   for (int s = 0; s < K / 16; ++s) {
     const uint64_t ad = smem_desc(a_saddr + s * a_step, a_lbo, a_sbo);
     const uint64_t bd = smem_desc(b_saddr + s * b_step, b_lbo, b_sbo);
     mma_bf16(d_tmem, ad, bd, idesc, (accumulate || s > 0) ? 1u : 0u);
   }
+}
+// gemm_steps, then a commit to *bar.
+__device__ __forceinline__ void gemm_issue(uint32_t d_tmem, uint32_t a_saddr, uint32_t a_lbo,
+                                           uint32_t a_sbo, uint32_t a_step, uint32_t b_saddr,
+                                           uint32_t b_lbo, uint32_t b_sbo, uint32_t b_step,
+                                           uint32_t idesc, int K, bool accumulate,
+                                           uint64_t *bar) {
+  gemm_steps(d_tmem, a_saddr, a_lbo, a_sbo, a_step, b_saddr, b_lbo, b_sbo, b_step, idesc, K,
+             accumulate);
   mma_commit(bar);
 }
 
