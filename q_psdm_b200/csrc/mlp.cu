@@ -20,18 +20,20 @@
 // samples); with two teams the queue ran dry while both waited for their MMAs:
 // 5.96 ms, three teams and biases read four to a load: 4.98 ms.
 //
-// Training: one team of 16 warps per CTA, 32 columns to a thread.  Backward forms
-//   dW_l = dZ_l^T H_{l-1}   (A = dZ MN-major view, B = H MN-major view)
-//   dH_{l-1} = dZ_l W_l      (A = dZ K-major, B = W MN-major view)
-// from what forward left in place: Z2 and Z3 in tensor memory, Z4 in
-// registers, H1..H3 in shared memory next to the weights, H4 where W2 lies
-// (W2 is read again from L2 for the last product).  dZ_l takes the buffer of
-// H_l, whose last reader is done by then.
+// Training: one team of 16 warps per CTA, everything transposed: TMEM lanes
+// are features, columns the T samples of a tile (64 or 128), T / 4 of them to a
+// thread.  Activations are kept as [feature][sample], which the products read
+// either way round:
+//   Z_l^T = W_l H_{l-1}^T     dH_{l-1}^T = W_l^T dZ_l^T     dW_l = dZ_l^T H_{l-1}
+// A thread's bias is one number and its part of a bias gradient a sum over its
+// own registers.  Backward works from what forward left in place: Z2 and Z3 in
+// tensor memory, Z4 in registers, H1..H4 in shared memory (for T = 128 H4 lies
+// where W2 is, which is read again from L2 for the last product).  dZ_l takes
+// the buffer of H_l, whose last reader is done by then.
 // Each CTA writes its gradients to its own slice of a global buffer (the first
-// tile's are stored, further ones added: plain, no atomics); bias gradients
-// are reduced across a warp by a butterfly transpose-sum and across warps in a
-// fixed order; one kernel then sums the slices in a fixed order, does the Adam
-// step and writes the BF16 images, so training is deterministic.
+// tile's are stored, further ones added: plain, no atomics); one kernel then
+// sums the slices in a fixed order, does the Adam step and writes the BF16
+// images, so training is deterministic.
 //
 // SiLU(z) = z sigma(z) = h + h tanh(h), h = z / 2, with the hardware FP32
 // tanh (tanh.approx.f32, about 2^-11 relative, below the BF16 rounding of
@@ -41,6 +43,7 @@
 #include <cuda_bf16.h>
 #include <math.h>
 
+#include <algorithm>
 #include <mutex>
 #include <utility>
 #include <vector>
@@ -71,18 +74,23 @@ constexpr int kXBytes = kTile * kIn * 2, kHBytes = kTile * kH * 2;
 // h = (z + b) / 2), then b5
 constexpr int kBiasBytes = (4 * kH + kOut) * 4;  // 2112
 constexpr int kGradThreads = 512;
-// training shared memory map
-constexpr int sX = kWBytes;                   // [128][16] bf16
-constexpr int sY = sX + kXBytes;              // dZ5, [128][16] bf16
-constexpr int sH1 = sY + kXBytes;             // H1, then dZ1: [128][128] bf16
-constexpr int sH2 = sH1 + kHBytes;            // H2, then dZ2
-constexpr int sH3 = sH2 + kHBytes;            // H3, then dZ3
-constexpr int sH4 = sW2;                      // H4, then dZ4, then W2 again
-constexpr int sBias = sH3 + kHBytes;
-constexpr int sDb = sBias + kBiasBytes;       // fp32 bias-gradient partials [4][4 quarters][128]
-constexpr int sDb5 = sDb + 16 * kH * 4;       // of layer 5: [4 quarters][16]
-constexpr int sLoss = sDb5 + 4 * kOut * 4;    // fp32 loss partials [16 warps]
-constexpr int kSmem = sLoss + 64;             // 223,616 bytes
+// training shared memory map for tiles of T samples
+template <int T>
+struct GradMap {
+  static constexpr int xb = T * kIn * 2, hb = T * kH * 2;
+  static constexpr int X = kWBytes;        // [T][16] bf16
+  static constexpr int Y = X + xb;         // dZ5, [T][16] bf16
+  static constexpr int H1 = Y + xb;        // H1^T, then dZ1^T: [128][T] bf16
+  static constexpr int H2 = H1 + hb;       // H2^T, then dZ2^T
+  static constexpr int H3 = H2 + hb;       // H3^T, then dZ3^T
+  static constexpr bool in_w2 = T > 64;    // H4 in place of W2
+  static constexpr int H4 = in_w2 ? sW2 : H3 + hb;
+  static constexpr int bias = H3 + (in_w2 ? 1 : 2) * hb;
+  static constexpr int db = bias + kBiasBytes;     // fp32 bias-gradient partials [4][4 parts][128]
+  static constexpr int db5 = db + 16 * kH * 4;     // of layer 5: [T / 32][16]
+  static constexpr int loss = db5 + 4 * kOut * 4;  // fp32 loss partials [16 warps]
+  static constexpr int bytes = loss + 64;          // 186,752 (T = 64), 223,616 (T = 128)
+};
 // inference shared memory map: weights, biases, then per team X and H
 constexpr int kFwdTeams = 3;
 constexpr int fBias = kWBytes;
@@ -203,48 +211,39 @@ struct Gemm {
   }
 };
 
-// 32 accumulator columns [c0, c0+32) of this thread's row.
-__device__ __forceinline__ void acc_ld32(uint32_t acc, const Role &ro, int c0, float *v) {
-  uint32_t r[32];
-  tc::tmem_ld16_nowait(acc + ro.lane_base + c0, r);
-  tc::tmem_ld16_nowait(acc + ro.lane_base + c0 + 16, r + 16);
-  tc::tmem_wait_ld_dep16(r);
-  tc::tmem_wait_ld_dep16(r + 16);
+// N accumulator columns [c0, c0+N) of this thread's row.
+template <int N>
+__device__ __forceinline__ void acc_ld(uint32_t acc, const Role &ro, int c0, float *v) {
+  uint32_t r[N];
 #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-__device__ __forceinline__ void acc_ld16(uint32_t acc, const Role &ro, int c0, float *v) {
-  tc::tmem_ld16(acc + ro.lane_base + c0, v);
+  for (int k = 0; k < N; k += 16) tc::tmem_ld16_nowait(acc + ro.lane_base + c0 + k, r + k);
+#pragma unroll
+  for (int k = 0; k < N; k += 16) tc::tmem_wait_ld_dep16(r + k);
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// H = SiLU(z + b) of 32 columns from c0 on, into a [128][128] buffer.  The
+// H = SiLU(acc + b) for this thread's 64 columns, into a [128][128] buffer, 32
+// columns at a time (80 registers hold three teams of 256 threads an SM).  The
 // biases are read four to a load: with one each, they were half of the
 // epilogue's instructions to the shared-memory and special-function queue.
-__device__ __forceinline__ void silu_row32(const float *z, const Role &ro, int c0,
-                                           const float *hb, uint8_t *hout) {
-  float v[32];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const float4 b = *reinterpret_cast<const float4 *>(hb + c0 + 4 * i);
-    v[4 * i] = silu_h(fmaf(0.5f, z[4 * i], b.x));
-    v[4 * i + 1] = silu_h(fmaf(0.5f, z[4 * i + 1], b.y));
-    v[4 * i + 2] = silu_h(fmaf(0.5f, z[4 * i + 2], b.z));
-    v[4 * i + 3] = silu_h(fmaf(0.5f, z[4 * i + 3], b.w));
-  }
-#pragma unroll
-  for (int k = 0; k < 4; ++k) st_row8(hout, ro.row, c0 + 8 * k, kH, v + 8 * k);
-}
-// H = SiLU(acc + b) for this thread's COLS columns, 32 at a time (80 registers
-// hold three teams of 256 threads an SM).
-template <int COLS>
 __device__ __forceinline__ void epi_silu(uint32_t acc, const Role &ro, const float *hb,
                                          uint8_t *hout) {
 #pragma unroll
-  for (int h = 0; h < COLS / 32; ++h) {
-    const int c0 = ro.part * COLS + 32 * h;
-    float z[32];
-    acc_ld32(acc, ro, c0, z);
-    silu_row32(z, ro, c0, hb, hout);
+  for (int h = 0; h < 2; ++h) {
+    const int c0 = ro.part * 64 + 32 * h;
+    float v[32];
+    acc_ld<32>(acc, ro, c0, v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float4 b = *reinterpret_cast<const float4 *>(hb + c0 + 4 * i);
+      v[4 * i] = silu_h(fmaf(0.5f, v[4 * i], b.x));
+      v[4 * i + 1] = silu_h(fmaf(0.5f, v[4 * i + 1], b.y));
+      v[4 * i + 2] = silu_h(fmaf(0.5f, v[4 * i + 2], b.z));
+      v[4 * i + 3] = silu_h(fmaf(0.5f, v[4 * i + 3], b.w));
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) st_row8(hout, ro.row, c0 + 8 * k, kH, v + 8 * k);
   }
 }
 
@@ -272,20 +271,26 @@ __device__ __forceinline__ void put_x(uint8_t *sx, int row, const float *__restr
   put_raw(sx, row, raw, live, ta);
 }
 
-// Copy weights (bf16 images) and biases (half biases for layers 1-4).
+// Copy weights (bf16 images) and biases (half biases for layers 1-4); NT threads.
+template <int NT>
 __device__ __forceinline__ void load_weights(uint8_t *sm, float *bias,
                                              const uint8_t *__restrict__ wimg,
                                              const float *__restrict__ params) {
   const uint4 *src = reinterpret_cast<const uint4 *>(wimg);
   uint4 *dst = reinterpret_cast<uint4 *>(sm);
-  for (int i = threadIdx.x; i < kWBytes / 16; i += blockDim.x) dst[i] = src[i];
-  for (int i = threadIdx.x; i < kH; i += blockDim.x) {
-    bias[i] = 0.5f * params[oB1 + i];
-    bias[kH + i] = 0.5f * params[oB2 + i];
-    bias[2 * kH + i] = 0.5f * params[oB3 + i];
-    bias[3 * kH + i] = 0.5f * params[oB4 + i];
+  constexpr int kN = kWBytes / 16;
+  uint4 w[(kN + NT - 1) / NT];
+#pragma unroll
+  for (int i = 0; i < (kN + NT - 1) / NT; ++i)
+    if (i * NT + (int)threadIdx.x < kN) w[i] = src[i * NT + threadIdx.x];
+  for (int i = threadIdx.x; i < 4 * kH; i += NT) {
+    const int l = i / kH;
+    bias[i] = 0.5f * params[(l == 0 ? oB1 : l == 1 ? oB2 : l == 2 ? oB3 : oB4) + i % kH];
   }
   if (threadIdx.x < kOut) bias[4 * kH + threadIdx.x] = params[oB5 + threadIdx.x];
+#pragma unroll
+  for (int i = 0; i < (kN + NT - 1) / NT; ++i)
+    if (i * NT + (int)threadIdx.x < kN) dst[i * NT + threadIdx.x] = w[i];
 }
 
 // ---------------------------------------------------------------------------
@@ -305,7 +310,7 @@ __global__ void __launch_bounds__(kFwdTeams * kTeam, 1)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   float *bias = reinterpret_cast<float *>(sm + fBias);
-  load_weights(sm, bias, wimg, params);
+  load_weights<kFwdTeams * kTeam>(sm, bias, wimg, params);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -330,16 +335,16 @@ __global__ void __launch_bounds__(kFwdTeams * kTeam, 1)
       load_raw(x, s + ahead, s < nsamp - ahead, raw);
     }
     if (!g.run(acc, sx, kIn, 0, sm + sW1, kIn, 0, kH, kIn)) break;
-    epi_silu<64>(acc, ro, bias, sh);
+    epi_silu(acc, ro, bias, sh);
     bool ok = true;
     for (int l = 1; l < 4 && ok; ++l) {
       ok = g.run(acc, sh, kH, 0, sm + sW2 + (l - 1) * kH * kH * 2, kH, 0, kH, kH);
-      if (ok) epi_silu<64>(acc, ro, bias + l * kH, sh);
+      if (ok) epi_silu(acc, ro, bias + l * kH, sh);
     }
     if (!ok || !g.run(acc, sh, kH, 0, sm + sW5, kH, 0, kOut, kH)) break;
     if (ro.part == 0) {
       float v[16];
-      acc_ld16(acc, ro, 0, v);
+      acc_ld<16>(acc, ro, 0, v);
       if (live && !g.failed) {
         y[(size_t)s * 2] = v[0] + bias[4 * kH];
         y[(size_t)s * 2 + 1] = v[1] + bias[4 * kH + 1];
@@ -354,46 +359,35 @@ __global__ void __launch_bounds__(kFwdTeams * kTeam, 1)
 // ---------------------------------------------------------------------------
 // training
 // ---------------------------------------------------------------------------
-// Butterfly transpose-sum of 32 per-lane values over the warp: afterwards
-// lane l holds in v[0] the sum of column l (fixed order).
-template <int O>
-__device__ __forceinline__ void xsum_step(float *v, int lane) {
-  const bool up = (lane & O) != 0;
+// H^T = SiLU(z + b) of this thread's feature for samples c0..c0+N-1, into a
+// [128][T] buffer.
+template <int T, int N>
+__device__ __forceinline__ void put_silu(const float *z, const Role &ro, float hb, uint8_t *out) {
+  const int c0 = ro.part * N;
+  float v[N];
 #pragma unroll
-  for (int i = 0; i < O; ++i) {
-    const float send = up ? v[i] : v[i + O];
-    const float keep = up ? v[i + O] : v[i];
-    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, O);
-  }
-}
-__device__ __forceinline__ void xsum32(float *v, int lane) {
-  xsum_step<16>(v, lane);
-  xsum_step<8>(v, lane);
-  xsum_step<4>(v, lane);
-  xsum_step<2>(v, lane);
-  xsum_step<1>(v, lane);
+  for (int i = 0; i < N; ++i) v[i] = silu_h(fmaf(0.5f, z[i], hb));
+#pragma unroll
+  for (int k = 0; k < N / 8; ++k) st_row8(out, ro.row, c0 + 8 * k, T, v + 8 * k);
 }
 
-// dZ = dH (acc) * SiLU'(z + b) into a [128][128] buffer for this thread's 32
-// columns; this warp's bias-gradient partials (its 32 rows) into
-// db[quarter][column].
-__device__ __forceinline__ void dz_epilogue(const float *z, uint32_t acc, const Role &ro,
-                                            const float *hb, uint8_t *out, float *db, bool live) {
-  const int c0 = ro.part * 32;
-  float d[32];
-  acc_ld32(acc, ro, c0, d);
+// dZ^T = dH^T (acc) * SiLU'(z + b) into a [128][T] buffer; this thread's sum
+// (pairs of pairs) into db[part][feature].  A dead sample's dH is 0.
+template <int T, int N>
+__device__ __forceinline__ void put_dz(const float *z, uint32_t acc, const Role &ro, float hb,
+                                       uint8_t *out, float *db) {
+  const int c0 = ro.part * N;
+  float d[N];
+  acc_ld<N>(acc, ro, c0, d);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const float4 b = *reinterpret_cast<const float4 *>(hb + c0 + 4 * i);
-    d[4 * i] = live ? d[4 * i] * silu_grad_h(fmaf(0.5f, z[4 * i], b.x)) : 0.0f;
-    d[4 * i + 1] = live ? d[4 * i + 1] * silu_grad_h(fmaf(0.5f, z[4 * i + 1], b.y)) : 0.0f;
-    d[4 * i + 2] = live ? d[4 * i + 2] * silu_grad_h(fmaf(0.5f, z[4 * i + 2], b.z)) : 0.0f;
-    d[4 * i + 3] = live ? d[4 * i + 3] * silu_grad_h(fmaf(0.5f, z[4 * i + 3], b.w)) : 0.0f;
-  }
+  for (int i = 0; i < N; ++i) d[i] = d[i] * silu_grad_h(fmaf(0.5f, z[i], hb));
 #pragma unroll
-  for (int k = 0; k < 4; ++k) st_row8(out, ro.row, c0 + 8 * k, kH, d + 8 * k);
-  xsum32(d, ro.lane);
-  db[ro.quarter * kH + c0 + ro.lane] = d[0];
+  for (int k = 0; k < N / 8; ++k) st_row8(out, ro.row, c0 + 8 * k, T, d + 8 * k);
+#pragma unroll
+  for (int o = N / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < o; ++i) d[i] += d[i + o];
+  db[ro.part * kH + ro.row] = d[0];
 }
 
 // Order of a weight block [128][K] in a gradient slice: [K / 4][128][4], so that a
@@ -414,23 +408,29 @@ __device__ __forceinline__ void put_grad4(float *gs, int off, int row, int c, co
 __device__ __forceinline__ void put_grad128(uint32_t acc, const Role &ro, float *gs, int off,
                                             bool first) {
   float v[32];
-  acc_ld32(acc, ro, ro.part * 32, v);
+  acc_ld<32>(acc, ro, ro.part * 32, v);
 #pragma unroll
   for (int k = 0; k < 8; ++k) put_grad4(gs, off, ro.row, ro.part * 32 + 4 * k, v + 4 * k, first);
 }
 
 // x: [n][5], t: [n][2]; grads: [gridDim.x][kSlice]
 //
-// One tile is a chain of ten tile products and the epilogues between them, and
-// at the usual batch (64 tiles of 8,192 samples) a CTA has one tile: latency
-// bounds it.  So the chain is kept short (nothing is computed twice but Z1,
-// products that are ready together are committed together), 512 threads halve
-// each epilogue against 256, and gradient tiles are written out while the next
-// products run.  8,192 samples: 85.7 us before, @GRAD@ us now.
+// One tile is a chain of ten waits for tile products with the epilogues between
+// them, and at the usual batch a CTA has one tile: latency bounds it.  So the
+// chain is kept short (nothing is computed twice but Z1, products that are ready
+// together are committed together), 512 threads share each epilogue, gradient
+// tiles are written out while the next products run, and tiles of 64 samples
+// are taken while one per SM is enough (grad_tile below).
+// 8,192 samples: 85.7 us before, 33 us with the short chain on tiles of 128
+// samples as rows, 16.7 us transposed on 128 tiles of 64 (25,000 cycles: 3,600
+// to load the weights, 900 per wait for a 128-deep product, 2,000 per gradient tile).
+template <int T>
 __global__ void __launch_bounds__(kGradThreads, 1)
     k_mlp_grad(const uint8_t *__restrict__ wimg, const float *__restrict__ params,
                const float *__restrict__ x, const float *__restrict__ t, int nsamp,
                MlpTileArgs ta, float *__restrict__ grads, int *err) {
+  using M = GradMap<T>;
+  constexpr int N = T / 4;  // samples to a thread
   extern __shared__ __align__(1024) uint8_t sm[];
   __shared__ uint64_t bar;
   __shared__ uint32_t tslot;
@@ -441,46 +441,54 @@ __global__ void __launch_bounds__(kGradThreads, 1)
     tc::mbar_init(&bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  const float *bias = reinterpret_cast<const float *>(sm + sBias);
-  load_weights(sm, reinterpret_cast<float *>(sm + sBias), wimg, params);
+  float *bias = reinterpret_cast<float *>(sm + M::bias);
+  load_weights<kGradThreads>(sm, bias, wimg, params);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   // tensor memory: accumulators A..D of 128 columns each
   const uint32_t tA = tslot, tB = tslot + 128, tC = tslot + 256, tD = tslot + 384;
   const Role ro(tid);
-  const int c0 = ro.part * 32;
+  const int c0 = ro.part * N;
+  const bool sample = ro.part == 0 && ro.row < T;  // this thread reads and writes a sample
+  const float hb1 = bias[ro.row], hb2 = bias[kH + ro.row], hb3 = bias[2 * kH + ro.row],
+              hb4 = bias[3 * kH + ro.row];
   Gemm g{Team{1u, kGradThreads}, &bar, 0u, err, tid == 0, false};
-  float *db = reinterpret_cast<float *>(sm + sDb), *db5 = reinterpret_cast<float *>(sm + sDb5);
+  float *db = reinterpret_cast<float *>(sm + M::db), *db5 = reinterpret_cast<float *>(sm + M::db5);
   float loss = 0.0f;
-  const int ntiles = (nsamp + kTile - 1) / kTile;
+  const int ntiles = (nsamp + T - 1) / T;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int s = tile * kTile + ro.row;
+    const int s = tile * T + ro.row;
     const bool live = s < nsamp, first = tile == blockIdx.x;
     float t0 = 0.0f, t1 = 0.0f;
-    if (ro.part == 0) {
-      put_x(sm + sX, ro.row, x, s, live, ta);
+    if (sample) {
+      put_x(sm + M::X, ro.row, x, s, live, ta);
       if (live) {
         t0 = __ldg(t + (size_t)s * 2);
         t1 = __ldg(t + (size_t)s * 2 + 1);
       }
     }
     // forward: Z1 in A, Z2 in B, Z3 in C, Z4 in registers, Y in A
-    if (!g.run(tA, sm + sX, kIn, 0, sm + sW1, kIn, 0, kH, kIn)) break;
-    epi_silu<32>(tA, ro, bias, sm + sH1);
-    if (!g.run(tB, sm + sH1, kH, 0, sm + sW2, kH, 0, kH, kH)) break;
-    epi_silu<32>(tB, ro, bias + kH, sm + sH2);
-    if (!g.run(tC, sm + sH2, kH, 0, sm + sW3, kH, 0, kH, kH)) break;
-    epi_silu<32>(tC, ro, bias + 2 * kH, sm + sH3);
-    if (!g.run(tD, sm + sH3, kH, 0, sm + sW4, kH, 0, kH, kH)) break;
-    float z[32];
-    acc_ld32(tD, ro, c0, z);
-    silu_row32(z, ro, c0, bias + 3 * kH, sm + sH4);
-    if (!g.run(tA, sm + sH4, kH, 0, sm + sW5, kH, 0, kOut, kH)) break;
+    float z[N];
+    if (!g.run(tA, sm + sW1, kIn, 0, sm + M::X, kIn, 0, T, kIn)) break;
+    acc_ld<N>(tA, ro, c0, z);
+    put_silu<T, N>(z, ro, hb1, sm + M::H1);
+    if (!g.run(tB, sm + sW2, kH, 0, sm + M::H1, T, 1, T, kH)) break;
+    acc_ld<N>(tB, ro, c0, z);
+    put_silu<T, N>(z, ro, hb2, sm + M::H2);
+    if (!g.run(tC, sm + sW3, kH, 0, sm + M::H2, T, 1, T, kH)) break;
+    acc_ld<N>(tC, ro, c0, z);
+    put_silu<T, N>(z, ro, hb3, sm + M::H3);
+    if (!g.run(tD, sm + sW4, kH, 0, sm + M::H3, T, 1, T, kH)) break;
+    acc_ld<N>(tD, ro, c0, z);
+    put_silu<T, N>(z, ro, hb4, sm + M::H4);
+    // Y: lanes are samples here; of a 64-sample tile the upper 64 lanes come
+    // from what lies behind (at most 1 KB past H4, inside the block) and are not used
+    if (!g.run(tA, sm + M::H4, T, 1, sm + sW5, kH, 0, kOut, kH)) break;
     // loss and dZ5 = dY (2 live columns of 16)
-    if (ro.part == 0) {
+    if (sample) {
       float v[16], d5[16];
-      acc_ld16(tA, ro, 0, v);
+      acc_ld<16>(tA, ro, 0, v);
 #pragma unroll
       for (int j = 0; j < 16; ++j) d5[j] = 0.0f;
       if (live) {
@@ -490,8 +498,8 @@ __global__ void __launch_bounds__(kGradThreads, 1)
         d5[0] = 2.0f * ta.w_out[0] * e0 * ta.inv_batch;
         d5[1] = 2.0f * ta.w_out[1] * e1 * ta.inv_batch;
       }
-      st_row8(sm + sY, ro.row, 0, kOut, d5);
-      st_row8(sm + sY, ro.row, 8, kOut, d5 + 8);
+      st_row8(sm + M::Y, ro.row, 0, kOut, d5);
+      st_row8(sm + M::Y, ro.row, 8, kOut, d5 + 8);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         float a = d5[j];
@@ -500,69 +508,73 @@ __global__ void __launch_bounds__(kGradThreads, 1)
       }
       if (ro.lane < kOut - 2) db5[ro.quarter * kOut + 2 + ro.lane] = 0.0f;
     }
-    // layer 5: dW5^T = H4^T dZ5 (rows = in), dH4 = dZ5 W5
+    // layer 5: dH4^T = W5^T dZ5^T, dW5^T = H4^T dZ5 (rows = in)
     if (!g.begin()) break;
     if (g.leader) {
-      g.add(tD, sm + sY, kOut, 0, sm + sW5, kH, 1, kH, kOut);
-      g.add(tA, sm + sH4, kH, 1, sm + sY, kOut, 1, kOut, kTile);
+      g.add(tD, sm + sW5, kH, 1, sm + M::Y, kOut, 0, T, kOut);
+      g.add(tA, sm + M::H4, T, 0, sm + M::Y, kOut, 1, kOut, T);
       g.commit();
     }
     g.finish();
     if (ro.part == 0) {
       float v[16];
-      acc_ld16(tA, ro, 0, v);
+      acc_ld<16>(tA, ro, 0, v);
 #pragma unroll
       for (int j = 0; j < kOut; ++j) {
         float *p = gs + oW5 + j * kH + ro.row;
         *p = first ? v[j] : *p + v[j];
       }
     }
-    dz_epilogue(z, tD, ro, bias + 3 * kH, sm + sH4, db + 12 * kH, live);
+    put_dz<T, N>(z, tD, ro, hb4, sm + M::H4, db + 12 * kH);
     // layer 4
     if (!g.begin()) break;
     if (g.leader) {
-      g.add(tD, sm + sH4, kH, 0, sm + sW4, kH, 1, kH, kH);
-      g.add(tA, sm + sH4, kH, 1, sm + sH3, kH, 1, kH, kTile);
+      g.add(tD, sm + sW4, kH, 1, sm + M::H4, T, 1, T, kH);
+      g.add(tA, sm + M::H4, T, 0, sm + M::H3, T, 0, kH, T);
       g.commit();
     }
-    // W2 back from L2 (its place is free once these products are done)
-    uint4 w2[kHBytes / 16 / kGradThreads];
+    if constexpr (M::in_w2) {
+      // W2 back from L2 (its place is free once these products are done)
+      uint4 w2[kHBytes / 16 / kGradThreads];
 #pragma unroll
-    for (int i = 0; i < kHBytes / 16 / kGradThreads; ++i)
-      w2[i] = __ldg(reinterpret_cast<const uint4 *>(wimg + sW2) + i * kGradThreads + tid);
-    g.finish();
+      for (int i = 0; i < kHBytes / 16 / kGradThreads; ++i)
+        w2[i] = __ldg(reinterpret_cast<const uint4 *>(wimg + sW2) + i * kGradThreads + tid);
+      g.finish();
 #pragma unroll
-    for (int i = 0; i < kHBytes / 16 / kGradThreads; ++i)
-      reinterpret_cast<uint4 *>(sm + sW2)[i * kGradThreads + tid] = w2[i];
-    acc_ld32(tC, ro, c0, z);
-    dz_epilogue(z, tD, ro, bias + 2 * kH, sm + sH3, db + 8 * kH, live);
+      for (int i = 0; i < kHBytes / 16 / kGradThreads; ++i)
+        reinterpret_cast<uint4 *>(sm + sW2)[i * kGradThreads + tid] = w2[i];
+    } else {
+      g.finish();
+    }
+    acc_ld<N>(tC, ro, c0, z);
+    put_dz<T, N>(z, tD, ro, hb3, sm + M::H3, db + 8 * kH);
     // layer 3; dW4 out meanwhile
     if (!g.begin()) break;
     if (g.leader) {
-      g.add(tD, sm + sH3, kH, 0, sm + sW3, kH, 1, kH, kH);
-      g.add(tC, sm + sH3, kH, 1, sm + sH2, kH, 1, kH, kTile);
+      g.add(tD, sm + sW3, kH, 1, sm + M::H3, T, 1, T, kH);
+      g.add(tC, sm + M::H3, T, 0, sm + M::H2, T, 0, kH, T);
       g.commit();
     }
     put_grad128(tA, ro, gs, oW4, first);
     g.finish();
-    acc_ld32(tB, ro, c0, z);
-    dz_epilogue(z, tD, ro, bias + kH, sm + sH2, db + 4 * kH, live);
+    acc_ld<N>(tB, ro, c0, z);
+    put_dz<T, N>(z, tD, ro, hb2, sm + M::H2, db + 4 * kH);
     // layer 2 and Z1 again; dW3 out meanwhile
     if (!g.begin()) break;
     if (g.leader) {
-      g.add(tD, sm + sH2, kH, 0, sm + sW2, kH, 1, kH, kH);
-      g.add(tA, sm + sX, kIn, 0, sm + sW1, kIn, 0, kH, kIn);
-      g.add(tB, sm + sH2, kH, 1, sm + sH1, kH, 1, kH, kTile);
+      g.add(tD, sm + sW2, kH, 1, sm + M::H2, T, 1, T, kH);
+      g.add(tA, sm + sW1, kIn, 0, sm + M::X, kIn, 0, T, kIn);
+      g.add(tB, sm + M::H2, T, 0, sm + M::H1, T, 0, kH, T);
       g.commit();
     }
     put_grad128(tC, ro, gs, oW3, first);
     g.finish();
-    acc_ld32(tA, ro, c0, z);
-    dz_epilogue(z, tD, ro, bias, sm + sH1, db, live);
-    // layer 1; dW2 and the bias gradients (four quarters in order) out meanwhile
+    acc_ld<N>(tA, ro, c0, z);
+    put_dz<T, N>(z, tD, ro, hb1, sm + M::H1, db);
+    // layer 1; dW2 and the bias gradients (parts in order) out meanwhile
     if (!g.begin()) break;
     if (g.leader) {
-      g.add(tC, sm + sH1, kH, 1, sm + sX, kIn, 1, kIn, kTile);
+      g.add(tC, sm + M::H1, T, 0, sm + M::X, kIn, 1, kIn, T);
       g.commit();
     }
     put_grad128(tB, ro, gs, oW2, first);
@@ -573,8 +585,8 @@ __global__ void __launch_bounds__(kGradThreads, 1)
       const float a = ((q[0] + q[kH]) + q[2 * kH]) + q[3 * kH];
       *p = first ? a : *p + a;
       if (tid < kOut) {
-        const float a5 =
-            ((db5[tid] + db5[kOut + tid]) + db5[2 * kOut + tid]) + db5[3 * kOut + tid];
+        float a5 = db5[tid];
+        for (int i = 1; i < T / 32; ++i) a5 += db5[i * kOut + tid];
         float *p5 = gs + oB5 + tid;
         *p5 = first ? a5 : *p5 + a5;
       }
@@ -582,20 +594,20 @@ __global__ void __launch_bounds__(kGradThreads, 1)
     g.finish();
     if (ro.part == 0) {
       float v[16];
-      acc_ld16(tC, ro, 0, v);
+      acc_ld<16>(tC, ro, 0, v);
 #pragma unroll
       for (int k = 0; k < 4; ++k) put_grad4(gs, oW1, ro.row, 4 * k, v + 4 * k, first);
     }
   }
   // loss sum of this CTA, in warp order
   for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-  float *ls = reinterpret_cast<float *>(sm + sLoss);
+  float *ls = reinterpret_cast<float *>(sm + M::loss);
   if (ro.lane == 0) ls[tid >> 5] = loss;
   tc::fence_before_sync();
   __syncthreads();
   if (tid == 0) {
     float a = 0.0f;
-    for (int w = 0; w < 4; ++w) a += ls[w];  // the warps of part 0
+    for (int w = 0; w < T / 32; ++w) a += ls[w];  // the warps that had samples
     *reinterpret_cast<float4 *>(gs + kParams) = make_float4(a * ta.inv_batch, 0.0f, 0.0f, 0.0f);
   }
   if (tid < 32) tc::tmem_free(tslot, 512);
@@ -654,8 +666,9 @@ __device__ __forceinline__ void adam1(float &p, float &m, float &v, float g, flo
 // then Adam on the FP32 master weights (padded entries are kept at zero) and
 // their BF16 images; only the loss goes to g.  Else the gradients go to g, in
 // parameter order.  The slices come from L2, up to 16 loads in flight a thread:
-// 64 slices (13.8 MB) with the update @UPD@ us, where the sum (one load in
-// flight), Adam and packing took 18.8 + 6.9 + 4.5 us as three launches.
+// 64 slices (13.8 MB) with the update 6.7 us (9.0 us for 128), where the sum
+// (one load in flight), Adam and packing took 18.8 + 6.9 + 4.5 us as three
+// launches; one thread to a sum took 9.6.
 constexpr int kUpdSums = 96, kUpdParts = 4;
 template <bool ADAM>
 __global__ void __launch_bounds__(kUpdSums * kUpdParts)
@@ -780,9 +793,29 @@ int mlp_device(const qpsdm_mlp *h) { return h->device; }
 
 constexpr int kUpdGrid = (kParams / 4 + 1 + kUpdSums - 1) / kUpdSums;
 
-static int mlp_grid(const qpsdm_mlp *h, int nsamp) {
-  const int ntiles = (nsamp + kTile - 1) / kTile;
-  return ntiles < h->nsm ? ntiles : h->nsm;
+// Gradient slices of n samples: tiles of 64 samples while every tile has an SM
+// of its own, since the epilogues of half a tile take half the time; else of
+// 128, which read the weights and write a slice half as often.  A step of 4,096
+// samples: 22.6 us with tiles of 64, 27.7 with 128; 8,192: 23.2 and 26.7;
+// 9,472 (the last that fits): 24.6 and 26.7.
+static int mlp_grad_tiles(const qpsdm_mlp *h, int n, bool *small) {
+  const int t64 = (n + 63) / 64, t128 = (n + 127) / 128;
+  *small = t64 <= h->nsm;
+  return *small ? t64 : std::min(t128, h->nsm);
+}
+static int mlp_grad_launch(const qpsdm_mlp *h, const float *d_x, const float *d_t, int n,
+                           cudaStream_t st) {
+  MlpTileArgs ta = h->ta;
+  ta.inv_batch = 1.0f / n;
+  bool small;
+  const int grid = mlp_grad_tiles(h, n, &small);
+  if (small)
+    k_mlp_grad<64><<<grid, kGradThreads, GradMap<64>::bytes, st>>>(h->wimg, h->p, d_x, d_t, n, ta,
+                                                                   h->slices, h->err);
+  else
+    k_mlp_grad<128><<<grid, kGradThreads, GradMap<128>::bytes, st>>>(
+        h->wimg, h->p, d_x, d_t, n, ta, h->slices, h->err);
+  return grid;
 }
 
 extern "C" int qpsdm_mlp_create(int device, qpsdm_mlp **out) {
@@ -823,8 +856,10 @@ extern "C" int qpsdm_mlp_create(int device, qpsdm_mlp **out) {
   cudaMemcpy(h->mask, mk.data(), sizeof(float) * kParams, cudaMemcpyHostToDevice);
   for (int j = 0; j < 5; ++j) h->ta.in_scale[j] = 1.0f;
   h->ta.w_out[0] = h->ta.w_out[1] = 1.0f;
-  if (cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) !=
-          cudaSuccess ||
+  if (cudaFuncSetAttribute(k_mlp_grad<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           GradMap<64>::bytes) != cudaSuccess ||
+      cudaFuncSetAttribute(k_mlp_grad<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           GradMap<128>::bytes) != cudaSuccess ||
       cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            kFwdSmem) != cudaSuccess) {
     qpsdm_mlp_destroy(h);
@@ -899,11 +934,7 @@ extern "C" int qpsdm_mlp_gradients(qpsdm_mlp *h, const float *d_x, const float *
   if (!h || !d_x || !d_t || n <= 0) return QPSDM_EINVAL;
   cudaSetDevice(h->device);
   cudaStream_t st = (cudaStream_t)stream;
-  MlpTileArgs ta = h->ta;
-  ta.inv_batch = 1.0f / n;
-  const int grid = mlp_grid(h, n);
-  k_mlp_grad<<<grid, kGradThreads, kSmem, st>>>(h->wimg, h->p, d_x, d_t, n, ta, h->slices,
-                                                h->err);
+  const int grid = mlp_grad_launch(h, d_x, d_t, n, st);
   k_mlp_update<false><<<kUpdGrid, kUpdSums * kUpdParts, 0, st>>>(h->slices, grid, h->p, h->m, h->v,
                                                         h->mask, AdamArgs{}, h->wimg, h->g);
   if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
@@ -921,11 +952,7 @@ extern "C" int qpsdm_mlp_train_step(qpsdm_mlp *h, const float *d_x, const float 
   if (!h || !d_x || !d_t || n <= 0 || !(lr > 0.0f)) return QPSDM_EINVAL;
   cudaSetDevice(h->device);
   cudaStream_t st = (cudaStream_t)stream;
-  MlpTileArgs ta = h->ta;
-  ta.inv_batch = 1.0f / n;
-  const int grid = mlp_grid(h, n);
-  k_mlp_grad<<<grid, kGradThreads, kSmem, st>>>(h->wimg, h->p, d_x, d_t, n, ta, h->slices,
-                                                h->err);
+  const int grid = mlp_grad_launch(h, d_x, d_t, n, st);
   h->step += 1;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.0f / (1.0f - powf(b1, (float)h->step));
