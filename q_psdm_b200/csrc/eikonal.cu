@@ -58,14 +58,34 @@ __device__ __forceinline__ float lin_grad_time(float r, float z, float v0, float
 // a block, two nodes a thread.  Only blocks that can change are visited: a
 // block whose nodes or facing neighbours changed in a sweep is on the next
 // sweep's list (a node's update depends on its six neighbours alone, so a
-// node left out would have kept its value).  Lists and the sweep a block was
-// last listed for live in the t* output until it is written.
+// node left out would have kept its value).  Lists, the sweep a block was last
+// listed for and the marks of blocks with start nodes (the only ones that sweep
+// 0 visits) live in the t* output until it is written.
 constexpr int kEx = 16, kEy = 8, kEz = 4, kEikThreads = kEx * kEy * kEz / 2;
+
+// n / d for n < 2^31 as a multiply-high and a shift: with 2^(l-1) < d <= 2^l,
+// mul = ceil(2^(31+l) / d) is exact (Granlund and Montgomery, "Division by
+// invariant integers using multiplication", 1994).
+struct EikDiv {
+  unsigned d, mul;
+  int shift;  // l - 1; unused for d = 1
+  EikDiv() = default;
+  explicit EikDiv(unsigned n) : d(n), mul(0), shift(0) {
+    int l = 0;
+    while ((1ull << l) < n) ++l;
+    if (n > 1) mul = (unsigned)(((1ull << (31 + l)) + n - 1) / n), shift = l - 1;
+  }
+  __device__ __forceinline__ int div(int n) const {
+    return d == 1 ? n : (int)(__umulhi((unsigned)n, mul) >> shift);
+  }
+};
 
 struct EikBlocks {
   qpsdm_eik_grid g;
   int nbx, nby, nbz, nblk;  // blocks per axis, blocks of all sources
-  int *list[2], *listed;    // [nblk] each
+  EikDiv row, plane, grid;  // by nbx, nbx nby, nbx nby nbz
+  int *list0, *list1;       // blocks of even and odd sweeps, [nblk] each
+  int *listed, *seed;       // sweep a block was last listed for; holds start nodes
   unsigned *count;          // list lengths of three consecutive sweeps, in turn
 };
 
@@ -75,12 +95,11 @@ struct EikBlock {
 };
 __device__ __forceinline__ EikBlock eik_block(const EikBlocks &B, int b) {
   EikBlock e;
-  const int per = B.nbx * B.nby * B.nbz;
-  e.s = b / per;
-  int r = b - e.s * per;
-  const int bz = r / (B.nbx * B.nby);
-  r -= bz * (B.nbx * B.nby);
-  const int by = r / B.nbx;
+  e.s = B.grid.div(b);
+  int r = b - e.s * (int)B.grid.d;
+  const int bz = B.plane.div(r);
+  r -= bz * (int)B.plane.d;
+  const int by = B.row.div(r);
   e.x0 = (r - by * B.nbx) * kEx;
   e.y0 = by * kEy;
   e.z0 = bz * kEz;
@@ -93,16 +112,16 @@ __device__ __forceinline__ void eik_mark(const EikBlocks &B, int b, const EikBlo
                                          unsigned faces, int sweep) {
   const int t = threadIdx.x;
   if (t > 6 || !((faces >> t) & 1u)) return;
-  const int step[3] = {1, B.nbx, B.nbx * B.nby};
-  const int at[3] = {e.x0 / kEx, e.y0 / kEy, e.z0 / kEz}, nb[3] = {B.nbx, B.nby, B.nbz};
   int o = b;
   if (t > 0) {
-    const int ax = (t - 1) >> 1, up = (t - 1) & 1;
-    if (up ? at[ax] + 1 >= nb[ax] : at[ax] == 0) return;
-    o += up ? step[ax] : -step[ax];
+    const int step = t < 3 ? 1 : t < 5 ? B.nbx : B.nbx * B.nby;
+    const int at = t < 3 ? e.x0 / kEx : t < 5 ? e.y0 / kEy : e.z0 / kEz;
+    const bool up = !(t & 1);
+    if (up ? at + 1 >= (t < 3 ? B.nbx : t < 5 ? B.nby : B.nbz) : at == 0) return;
+    o += up ? step : -step;
   }
   if (atomicExch(B.listed + o, sweep + 1) == sweep + 1) return;
-  B.list[(sweep + 1) & 1][atomicAdd(B.count + (sweep + 1) % 3, 1u)] = o;
+  (sweep & 1 ? B.list0 : B.list1)[atomicAdd(B.count + (sweep + 1) % 3, 1u)] = o;
 }
 // Which faces of its block a changed node lies on, and the block itself.
 __device__ __forceinline__ unsigned eik_faces(int lx, int ly, int lz) {
@@ -120,7 +139,7 @@ __global__ void k_eik_setup(const float *__restrict__ vel, const float *__restri
   if (blockIdx.x == 0 && threadIdx.x < 3) B.count[threadIdx.x] = 0;
   for (int b = blockIdx.x; b < B.nblk; b += gridDim.x) {
     const EikBlock e = eik_block(B, b);
-    if (threadIdx.x == 0) B.listed[b] = -1;
+    bool start = false;
     const float4 sp = src[e.s];  // source x, y; local grid origin ox, oy
     const float qs = model_at(invq, m, sp.x, sp.y, 0.0f);  // near-surface Q on the path
 #pragma unroll
@@ -139,69 +158,127 @@ __global__ void k_eik_setup(const float *__restrict__ vel, const float *__restri
         F[i] = -(g.h / v);
         T[i] = t;
         TS[i] = (double)t * qs;
+        start = true;
       } else {
         F[i] = g.h / v;
         T[i] = kInf;
         TS[i] = 0.0;
       }
     }
+    start = __syncthreads_or(start);
+    if (threadIdx.x == 0) {
+      B.listed[b] = -1;
+      B.seed[b] = start;
+    }
   }
 }
 
-// One in-place Godunov relaxation of the listed blocks (sweep 0: every block).
+// Godunov update of a node from the smaller neighbour value of each axis.
+__device__ __forceinline__ float eik_update(float a, float b, float c, float f) {
+  const float t0 = fminf(a, fminf(b, c)), t2 = fmaxf(a, fmaxf(b, c));
+  const float t1 = fminf(fmaxf(a, b), fmaxf(fminf(a, b), c));  // middle value
+  if (t0 >= kInf) return kInf;
+  float t = t0 + f;
+  if (t > t1 && t1 < kInf) {
+    const float s2 = t0 + t1, d2 = 2.0f * f * f - (t0 - t1) * (t0 - t1);
+    t = 0.5f * (s2 + sqrtf(fmaxf(d2, 0.0f)));
+    if (t > t2 && t2 < kInf) {
+      const float s3 = t0 + t1 + t2;
+      const float d3 = s3 * s3 - 3.0f * (t0 * t0 + t1 * t1 + t2 * t2 - f * f);
+      t = (s3 + sqrtf(fmaxf(d3, 0.0f))) / 3.0f;
+    }
+  }
+  return t;
+}
+
+// Godunov relaxation of the listed blocks (sweep 0: those with start nodes),
+// each with its halo in shared memory, red nodes and black nodes in turn (a
+// node's neighbours are all of the other colour: no node is read while it is
+// written), until
+// nothing changes, kEikInner times at most.  A thread has one node of each
+// colour, neighbours in x.  Rows of 24 words: a warp's 8 x 4 nodes of one
+// colour lie in 32 banks.
 //
-// Bound by issue (64 % active) and the loads' latency.  A sweep of all 28 M nodes
-// of 32 sources took 0.27 ms, with the 64-bit divisions of a flat node index,
-// and 256 sweeps 70 ms, although a block changes in about 60 of them: 15.4 ms
-// now.  (Listing a neighbour only where its value is the larger one took more
-// registers than it saved blocks: 23.5 ms.)
+// Bound by issue, and by the colours taking turns at a barrier.  28 M nodes, 32
+// sources: 256 sweeps over every node, in global memory, took 70 ms; over listed
+// blocks, one update a visit, 15.4 ms in 224 sweeps; now 5.4 ms in 80.  With 1,
+// 2, 4, 8, 16 updates a visit at most, and 7 ms of t* in each: 26.5, 20.8, 14.9,
+// 13.1, 12.9 ms.  Eight: the FP32 update's rounding lets values creep below the
+// fixed point, and the fewer updates, the less they do (error 0.6 to 1.3 of the
+// full sweeps', 0.98 on average); with 16 they end up to 4 times as far from the
+// full sweeps' values as two runs of those from each other, with 8 at most 3 times.
+constexpr int kEikInner = 8;
 __global__ void __launch_bounds__(kEikThreads)
     k_eik_relax(const float *__restrict__ F, float *__restrict__ T, EikBlocks B, int sweep) {
+  constexpr int HX = 24, HY = kEy + 2, HZ = kEz + 2;
+  __shared__ float s_t[HX * HY * HZ];
   __shared__ unsigned s_faces;
   const qpsdm_eik_grid g = B.g;
+  const size_t sxy = (size_t)g.nx * g.ny;
   const int n = sweep == 0 ? B.nblk : (int)B.count[sweep % 3];
   if (blockIdx.x == 0 && threadIdx.x == 0) B.count[(sweep + 2) % 3] = 0;
+  const int tid = threadIdx.x;
+  const int px = tid % (kEx / 2), ly = tid / (kEx / 2) % kEy, lz = tid / (kEx / 2 * kEy);
+  const int odd = (ly + lz) & 1;
+  // node c (0 red, 1 black) of this thread
+  const int lx[2] = {2 * px + odd, 2 * px + (odd ^ 1)};
+  const int row = ((lz + 1) * HY + ly + 1) * HX + 1;
   for (int k = blockIdx.x; k < n; k += gridDim.x) {
-    const int blk = sweep == 0 ? k : B.list[sweep & 1][k];
+    if (sweep == 0 && !B.seed[k]) continue;  // uniform in the CTA
+    const int blk = sweep == 0 ? k : (sweep & 1 ? B.list1 : B.list0)[k];
     const EikBlock e = eik_block(B, blk);
-    if (threadIdx.x == 0) s_faces = 0;
+    if (tid == 0) s_faces = 0;
+    const bool in_yz = e.y0 + ly < g.ny && e.z0 + lz < g.nz;
+    const size_t i0 = e.base + lz * sxy + (size_t)ly * g.nx;
+    float f[2], t[2], old[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const bool in = in_yz && e.x0 + lx[c] < g.nx;
+      f[c] = in ? F[i0 + lx[c]] : -kInf;
+      old[c] = t[c] = in ? T[i0 + lx[c]] : kInf;
+      s_t[row + lx[c]] = t[c];
+    }
+    // halo: z faces (two rows of 128), y faces (64 each), x faces (32 each)
+    auto halo = [&](int hx, int hy, int hz) {
+      const int x = e.x0 + hx, y = e.y0 + hy, z = e.z0 + hz;
+      const bool in = x >= 0 && x < g.nx && y >= 0 && y < g.ny && z >= 0 && z < g.nz;
+      s_t[((hz + 1) * HY + hy + 1) * HX + hx + 1] =
+          in ? T[e.base + hz * (ptrdiff_t)sxy + hy * (ptrdiff_t)g.nx + hx] : kInf;
+    };
+    halo(tid % kEx, tid / kEx % kEy, tid < 128 ? -1 : kEz);
+    if (tid < 128)
+      halo(tid % kEx, tid < 64 ? -1 : kEy, tid / kEx % kEz);
+    else if (tid < 192)
+      halo(tid < 160 ? -1 : kEx, tid % kEy, tid / kEy % kEz);
     __syncthreads();
+    bool more = true;
+    for (int it = 0; it < kEikInner && more; ++it) {
+      bool ch = false;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        if (f[c] >= 0.0f) {
+          const float *p = s_t + row + lx[c];
+          const float v = eik_update(fminf(p[-1], p[1]), fminf(p[-HX], p[HX]),
+                                     fminf(p[-HX * HY], p[HX * HY]), f[c]);
+          if (v < t[c] * (1.0f - 1e-7f)) {
+            t[c] = v;
+            s_t[row + lx[c]] = v;
+            ch = true;
+          }
+        }
+        if (c == 0) __syncthreads();
+      }
+      more = __syncthreads_or(ch);
+    }
     unsigned faces = 0;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int l = threadIdx.x + h * kEikThreads;
-      const int lx = l % kEx, ly = l / kEx % kEy, lz = l / (kEx * kEy);
-      const int ix = e.x0 + lx, iy = e.y0 + ly, iz = e.z0 + lz;
-      if (ix >= g.nx || iy >= g.ny || iz >= g.nz) continue;
-      const size_t sxy = (size_t)g.nx * g.ny;
-      const size_t i = e.base + lz * sxy + (size_t)ly * g.nx + lx;
-      const float f = F[i];
-      if (f < 0.0f) continue;
-      float a = kInf, b = kInf, c = kInf;
-      if (ix > 0) a = T[i - 1];
-      if (ix < g.nx - 1) a = fminf(a, T[i + 1]);
-      if (iy > 0) b = T[i - g.nx];
-      if (iy < g.ny - 1) b = fminf(b, T[i + g.nx]);
-      if (iz > 0) c = T[i - sxy];
-      if (iz < g.nz - 1) c = fminf(c, T[i + sxy]);
-      const float t0 = fminf(a, fminf(b, c)), t2 = fmaxf(a, fmaxf(b, c));
-      const float t1 = fminf(fmaxf(a, b), fmaxf(fminf(a, b), c));  // middle value
-      if (t0 >= kInf) continue;
-      float t = t0 + f;
-      if (t > t1 && t1 < kInf) {
-        const float s2 = t0 + t1, d2 = 2.0f * f * f - (t0 - t1) * (t0 - t1);
-        t = 0.5f * (s2 + sqrtf(fmaxf(d2, 0.0f)));
-        if (t > t2 && t2 < kInf) {
-          const float s3 = t0 + t1 + t2;
-          const float d3 = s3 * s3 - 3.0f * (t0 * t0 + t1 * t1 + t2 * t2 - f * f);
-          t = (s3 + sqrtf(fmaxf(d3, 0.0f))) / 3.0f;
-        }
-      }
-      if (t < T[i] * (1.0f - 1e-7f)) {
-        T[i] = t;
-        faces |= eik_faces(lx, ly, lz);
-      }
+    for (int c = 0; c < 2; ++c) {
+      if (t[c] < old[c]) T[i0 + lx[c]] = t[c];
+      // (sweep 0 lists what start nodes reach)
+      if (t[c] < old[c] || (sweep == 0 && f[c] < 0.0f && f[c] > -kInf))
+        faces |= eik_faces(lx[c], ly, lz) & ~1u;
     }
+    if (more) faces |= 1u;  // settled, unless the loop ran out
     if (faces) atomicOr(&s_faces, faces);
     __syncthreads();
     eik_mark(B, blk, e, s_faces, sweep);
@@ -214,14 +291,18 @@ __global__ void __launch_bounds__(kEikThreads)
 // it changes.  In sweep 0 the blocks that hold start nodes, and after it what
 // they reach: t* at a node depends on nodes of smaller T only, so the values
 // settle outwards from the source, most blocks in a few visits, and a block is
-// listed only for a changed neighbour of smaller T.  (256 sweeps over every
-// node took 95 ms for the 28 M nodes of 32 sources; 6.9 ms now.)
+// listed only for a changed neighbour of smaller T.  256 sweeps over every
+// node took 95 ms for the 28 M nodes of 32 sources; so 6.9 ms; 4.7 ms with the
+// traveltimes of the neighbours from shared memory, a halo of the facing nodes
+// only and the seed marks (a visit's preparation, not its FP64 updates, is most
+// of its instructions: three updates to a barrier gave nothing).
 constexpr int kTsThreads = kEx * kEy * kEz;
 __global__ void __launch_bounds__(kTsThreads)
     k_tstar_relax(const float *__restrict__ F, const float *__restrict__ T,
                   const float *__restrict__ QF, double *__restrict__ TS, EikBlocks B, int sweep) {
   constexpr int HX = kEx + 2, HY = kEy + 2, HZ = kEz + 2;
   __shared__ double s_ts[HX * HY * HZ];
+  __shared__ float s_t[HX * HY * HZ];
   __shared__ unsigned s_faces;
   const qpsdm_eik_grid g = B.g;
   const size_t sxy = (size_t)g.nx * g.ny;
@@ -230,28 +311,47 @@ __global__ void __launch_bounds__(kTsThreads)
   if (blockIdx.x == 0 && threadIdx.x == 0) B.count[(sweep + 2) % 3] = 0;
   const int lx = threadIdx.x % kEx, ly = threadIdx.x / kEx % kEy, lz = threadIdx.x / (kEx * kEy);
   const int at = ((lz + 1) * HY + ly + 1) * HX + lx + 1;
+  // this thread's node of the halo: z faces (128 each), y faces (64 each), x faces (32 each)
+  const int u = threadIdx.x;
+  int hx = -2, hy = 0, hz = 0;
+  if (u < 256)
+    hx = u % kEx, hy = u / kEx % kEy, hz = u < 128 ? -1 : kEz;
+  else if (u < 384)
+    hx = u % kEx, hy = u < 320 ? -1 : kEy, hz = u / kEx % kEz;
+  else if (u < 448)
+    hx = u < 416 ? -1 : kEx, hy = u % kEy, hz = u / kEy % kEz;
   for (int k = blockIdx.x; k < n; k += gridDim.x) {
-    const int blk = sweep == 0 ? k : B.list[sweep & 1][k];
+    if (sweep == 0 && !B.seed[k]) continue;  // uniform in the CTA
+    const int blk = sweep == 0 ? k : (sweep & 1 ? B.list1 : B.list0)[k];
     const EikBlock e = eik_block(B, blk);
-    const int ix = e.x0 + lx, iy = e.y0 + ly, iz = e.z0 + lz;
+    bool on = e.x0 + lx < g.nx && e.y0 + ly < g.ny && e.z0 + lz < g.nz;
     const size_t i = e.base + lz * sxy + (size_t)ly * g.nx + lx;
+    const bool start = on && F[i] < 0.0f;
+    if (threadIdx.x == 0) s_faces = 0;
+    // the block and the nodes facing it
+    const float ti = on ? T[i] : kInf;
+    const double old = on ? TS[i] : 0.0;
+    s_t[at] = ti;
+    s_ts[at] = old;
+    if (hx > -2) {
+      const int x = e.x0 + hx, y = e.y0 + hy, z = e.z0 + hz;
+      const bool in = x >= 0 && x < g.nx && y >= 0 && y < g.ny && z >= 0 && z < g.nz;
+      const ptrdiff_t o = hz * (ptrdiff_t)sxy + hy * (ptrdiff_t)g.nx + hx;
+      const int j = ((hz + 1) * HY + hy + 1) * HX + hx + 1;
+      s_t[j] = in ? T[e.base + o] : kInf;
+      s_ts[j] = in ? TS[e.base + o] : 0.0;
+    }
+    __syncthreads();
     // the update's terms: upwind neighbours and weights
     int nb[3] = {at, at, at};
-    double w[3] = {0.0, 0.0, 0.0}, q = 0.0, rden = 0.0, val = 0.0, old = 0.0;
+    double w[3] = {0.0, 0.0, 0.0}, q = 0.0, rden = 0.0, val = old;
     unsigned faces = 0;  // sides whose outside neighbour lies downwind
-    bool on = ix < g.nx && iy < g.ny && iz < g.nz, start = false;
     if (on) {
-      val = old = TS[i];
-      start = F[i] < 0.0f;
-      const float ti = T[i];
-      const size_t sd[3] = {1, (size_t)g.nx, sxy};
       const int hd[3] = {1, HX, HX * HY};
-      const int id[3] = {ix, iy, iz}, nd[3] = {g.nx, g.ny, g.nz};
       double den = 0.0;
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        const float lo = id[d] > 0 ? T[i - sd[d]] : kInf;
-        const float hi = id[d] < nd[d] - 1 ? T[i + sd[d]] : kInf;
+        const float lo = s_t[at - hd[d]], hi = s_t[at + hd[d]];
         const float best = fminf(lo, hi);
         if (best < ti) {
           w[d] = ((double)ti - (double)best) * ih2;
@@ -261,22 +361,12 @@ __global__ void __launch_bounds__(kTsThreads)
         faces |= (lo > ti ? 2u : 0u) << (2 * d) | (hi > ti ? 4u : 0u) << (2 * d);
       }
       faces &= eik_faces(lx, ly, lz);
-      q = QF[i];
       on = !start && ti < kInf && den > 0.0;
-      if (on) rden = 1.0 / den;
+      if (on) {
+        rden = 1.0 / den;
+        q = QF[i];
+      }
     }
-    if (threadIdx.x == 0) s_faces = 0;
-    const bool seed = __syncthreads_or(start);
-    if (sweep == 0 && !seed) continue;  // uniform in the CTA
-    for (int j = threadIdx.x; j < HX * HY * HZ; j += kTsThreads) {
-      const int hx = j % HX, hy = j / HX % HY, hz = j / (HX * HY);
-      const int jx = e.x0 + hx - 1, jy = e.y0 + hy - 1, jz = e.z0 + hz - 1;
-      const bool in = jx >= 0 && jx < g.nx && jy >= 0 && jy < g.ny && jz >= 0 && jz < g.nz;
-      s_ts[j] = in ? TS[e.base + (ptrdiff_t)(hz - 1) * (ptrdiff_t)sxy +
-                        (ptrdiff_t)(hy - 1) * g.nx + (hx - 1)]
-                   : 0.0;
-    }
-    __syncthreads();
     bool more = true;
     for (int it = 0; it < 64 && more; ++it) {
       bool ch = false;
@@ -391,10 +481,15 @@ extern "C" int qpsdm_eikonal_solve(const float *d_vel, const float *d_invq,
   const int64_t nblk = (int64_t)nsrc * B.nbx * B.nby * B.nbz;
   if (nblk > 0x7fffffff) return QPSDM_EINVAL;
   B.nblk = (int)nblk;
-  // a block has at least four nodes, so three words per block fit the output
-  B.list[0] = reinterpret_cast<int *>(d_tstar);
-  B.list[1] = B.list[0] + nblk;
-  B.listed = B.list[1] + nblk;
+  B.row = EikDiv(B.nbx);
+  B.plane = EikDiv(B.nbx * B.nby);
+  B.grid = EikDiv(B.nbx * B.nby * B.nbz);
+  // at least four nodes to a block (2, 1, 2 an axis: nx, nz >= 2), so four words
+  // per block fit the output
+  B.list0 = reinterpret_cast<int *>(d_tstar);
+  B.list1 = B.list0 + nblk;
+  B.listed = B.list1 + nblk;
+  B.seed = B.listed + nblk;
   B.count = reinterpret_cast<unsigned *>(TS + n);
   const float4 *src = (const float4 *)d_src;
   const int grd = (int)std::min<int64_t>(nblk, 148 * 8);
