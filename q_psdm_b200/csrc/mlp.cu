@@ -435,6 +435,9 @@ __global__ void __launch_bounds__(kGradThreads, 1)
   __shared__ uint64_t bar;
   __shared__ uint32_t tslot;
   const int tid = threadIdx.x;
+  // the update may be scheduled as soon as every CTA has started (it waits for
+  // the end of this kernel before it reads a slice)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   float *gs = grads + (size_t)blockIdx.x * kSlice;
   if (tid < 32) tc::tmem_alloc(&tslot, 512);
   if (tid == 0) {
@@ -687,6 +690,8 @@ __global__ void __launch_bounds__(kUpdSums * kUpdParts)
     m4 = *reinterpret_cast<float4 *>(m + o.p);
     v4 = *reinterpret_cast<float4 *>(v + o.p);
   }
+  // end of the gradient kernel: its slices, and its reads of p
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   // s == kParams: the loss, in the first of the slice's last 16 entries
   if (s <= kParams) {
     const int per = (nslice + kUpdParts - 1) / kUpdParts;
@@ -922,6 +927,26 @@ extern "C" int qpsdm_mlp_set_scaling(qpsdm_mlp *h, const float *in_shift, const 
   return QPSDM_OK;
 }
 
+// The update (or, without ADAM, the sum alone) behind its gradient kernel on
+// the stream, launched programmatically: its CTAs start and load their
+// parameters and moments while the last gradient CTAs run (k_mlp_grad writes none
+// of those).  A step of 8,192 samples 23.6 -> 21.7 us, of 4,096 22.6 -> 20.5.
+template <bool ADAM>
+static cudaError_t mlp_update_launch(qpsdm_mlp *h, int nslice, const AdamArgs &a,
+                                     cudaStream_t st) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(kUpdGrid);
+  c.blockDim = dim3(kUpdSums * kUpdParts);
+  c.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, k_mlp_update<ADAM>, (const float *)h->slices, nslice, h->p, h->m,
+                            h->v, (const float *)h->mask, a, h->wimg, h->g);
+}
+
 static int mlp_check_err(qpsdm_mlp *h) {
   int e = 0;
   if (cudaMemcpy(&e, h->err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
@@ -935,9 +960,9 @@ extern "C" int qpsdm_mlp_gradients(qpsdm_mlp *h, const float *d_x, const float *
   cudaSetDevice(h->device);
   cudaStream_t st = (cudaStream_t)stream;
   const int grid = mlp_grad_launch(h, d_x, d_t, n, st);
-  k_mlp_update<false><<<kUpdGrid, kUpdSums * kUpdParts, 0, st>>>(h->slices, grid, h->p, h->m, h->v,
-                                                        h->mask, AdamArgs{}, h->wimg, h->g);
-  if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
+  const cudaError_t ue = mlp_update_launch<false>(h, grid, AdamArgs{}, st);
+  if (ue != cudaSuccess || cudaGetLastError() != cudaSuccess ||
+      cudaStreamSynchronize(st) != cudaSuccess)
     return QPSDM_ECUDA;
   int rc = mlp_check_err(h);
   if (rc) return rc;
@@ -957,10 +982,9 @@ extern "C" int qpsdm_mlp_train_step(qpsdm_mlp *h, const float *d_x, const float 
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.0f / (1.0f - powf(b1, (float)h->step));
   const float c2 = 1.0f / (1.0f - powf(b2, (float)h->step));
-  k_mlp_update<true><<<kUpdGrid, kUpdSums * kUpdParts, 0, st>>>(
-      h->slices, grid, h->p, h->m, h->v, h->mask, AdamArgs{lr, b1, b2, 1e-8f, c1, c2}, h->wimg,
-      h->g);
-  if (cudaGetLastError() != cudaSuccess) return QPSDM_ECUDA;
+  const cudaError_t ue = mlp_update_launch<true>(
+      h, grid, AdamArgs{lr, b1, b2, 1e-8f, c1, c2}, st);
+  if (ue != cudaSuccess || cudaGetLastError() != cudaSuccess) return QPSDM_ECUDA;
   if (loss) {
     if (cudaMemcpyAsync(loss, h->g + kParams, sizeof(float), cudaMemcpyDeviceToHost, st) !=
             cudaSuccess ||
