@@ -1075,7 +1075,7 @@ def run_surrogate(dev, steps, warmup, n_query=1 << 22, batch=1 << 16):
                           "roofline": {"bound": "tensor", "achieved": tf_i, "peak": peak,
                                        "unit": "TFLOP/s", "frac": tf_i / peak,
                                        "flop_per_query": 2 * MLP_MAC, "peak_source": src}},
-            "training": {"kernels": "k_mlp_grad + k_mlp_reduce + k_mlp_adam + k_mlp_pack",
+            "training": {"kernels": "k_mlp_grad + k_mlp_update",
                          "batch": batch, "ms_per_step": ms_t,
                          "msamples_per_s": batch / ms_t / 1e3,
                          "roofline": {"bound": "tensor", "achieved": tf_t, "peak": peak,
