@@ -4,26 +4,25 @@
 // 16).  BF16 weights and activations, FP32 accumulation in tensor memory,
 // FP32 master weights and Adam moments in global memory.
 //
-// Every layer is one 128-sample tcgen05 tile GEMM (tc.cuh): activations are
-// the A operand ([sample][feature], K-major), weights [out][in] the B
-// operand, the FP32 accumulator 128 TMEM columns.  A team of 8 warps owns a
-// tile: warp w reads TMEM lane quarter (w mod 4) -- the quarter a warp may
-// access is fixed by its warp index -- and column half (w / 4), so the
-// epilogue of a layer (bias, SiLU, BF16 store) is spread over 256 threads.
+// Every layer is a tcgen05 tile product (tc.cuh) on BF16 operands in shared
+// memory, weights [out][in], with the FP32 accumulator in tensor memory.  Tiles
+// are held transposed: TMEM lanes are the 128 features, columns the samples,
+// and activations are kept as [feature][sample], which the products read
+// either way round.  Warp w reads TMEM lane quarter (w mod 4) -- the quarter a
+// warp may access is fixed by its warp index; a thread's bias is one number.
 //
-// Inference: three teams per CTA work on three tiles at once, each with its own
-// mbarrier, TMEM columns and activation buffer (a layer's output overwrites
-// its input once the MMA that read it has completed), so one team's MMAs run
-// while the others are in their epilogues.  Each thread loads its inputs of
-// the next tile while the current one is computed.  The special-function
-// queue bounds it (512 tanh a sample, 16 a cycle per SM: 3.0 ms for 26 M
-// samples); with two teams the queue ran dry while both waited for their MMAs:
-// 5.96 ms, three teams and biases read four to a load: 4.98 ms.
+// Inference: six teams of four warps per CTA work on six tiles of 64 samples at
+// once, each with its own mbarrier, TMEM columns and activation buffer (a layer's
+// output overwrites its input once the MMA that read it has completed), so
+// teams' MMAs run while others are in their epilogues.  Each thread loads its
+// inputs of the next tile while the current one is computed.  The
+// special-function queue bounds it (512 tanh a sample, 16 a cycle per SM: 3.0 ms
+// for 26 M samples).  It runs dry while teams wait for their MMAs together:
+// with two teams of eight warps, 128 samples as TMEM lanes and a load per bias
+// 5.96 ms, three teams and biases read four to a load 4.92 ms, now 4.08 ms.
 //
-// Training: one team of 16 warps per CTA, everything transposed: TMEM lanes
-// are features, columns the T samples of a tile (64 or 128), T / 4 of them to a
-// thread.  Activations are kept as [feature][sample], which the products read
-// either way round:
+// Training: one team of 16 warps per CTA, T = 64 or 128 samples to a tile, T / 4
+// of them to a thread:
 //   Z_l^T = W_l H_{l-1}^T     dH_{l-1}^T = W_l^T dZ_l^T     dW_l = dZ_l^T H_{l-1}
 // A thread's bias is one number and its part of a bias gradient a sum over its
 // own registers.  Backward works from what forward left in place: Z2 and Z3 in
@@ -55,7 +54,7 @@
 
 namespace qpsdm {
 
-constexpr int kH = 128, kIn = 16, kOut = 16, kTile = 128;
+constexpr int kH = 128, kIn = 16, kOut = 16;
 // FP32 parameter block offsets
 constexpr int oW1 = 0, oB1 = oW1 + kH * kIn;
 constexpr int oW2 = oB1 + kH, oB2 = oW2 + kH * kH;
@@ -68,8 +67,7 @@ constexpr int kSlice = kParams + 16;  // + loss sum and padding
 constexpr int sW1 = 0, sW2 = sW1 + kH * kIn * 2, sW3 = sW2 + kH * kH * 2;
 constexpr int sW4 = sW3 + kH * kH * 2, sW5 = sW4 + kH * kH * 2;
 constexpr int kWBytes = sW5 + kOut * kH * 2;  // 106496
-constexpr int kTeam = 256;                    // threads of a team
-constexpr int kXBytes = kTile * kIn * 2, kHBytes = kTile * kH * 2;
+constexpr int kHBytes = kH * kH * 2;          // a [128][128] block
 // biases in shared memory: half biases of layers 1-4 (the SiLU argument is
 // h = (z + b) / 2), then b5
 constexpr int kBiasBytes = (4 * kH + kOut) * 4;  // 2112
@@ -91,11 +89,13 @@ struct GradMap {
   static constexpr int loss = db5 + 4 * kOut * 4;  // fp32 loss partials [16 warps]
   static constexpr int bytes = loss + 64;          // 186,752 (T = 64), 223,616 (T = 128)
 };
-// inference shared memory map: weights, biases, then per team X and H
-constexpr int kFwdTeams = 3;
+// inference shared memory map: weights, biases, then per team X and H^T of a
+// tile; 1 KB behind the last (k_mlp_forward)
+constexpr int kFwdTile = 64, kFwdTeams = 6, kFwdTeam = 128;
+constexpr int kFwdTeamBytes = kFwdTile * (kIn + kH) * 2;
 constexpr int fBias = kWBytes;
 constexpr int fTeam0 = fBias + 2304;
-constexpr int kFwdSmem = fTeam0 + kFwdTeams * (kXBytes + kHBytes);  // 219,392 bytes
+constexpr int kFwdSmem = fTeam0 + kFwdTeams * kFwdTeamBytes + 1024;  // 220,416 bytes
 
 struct MlpTileArgs {
   float in_scale[5], in_shift[5];  // features = (raw - shift) * scale
@@ -223,30 +223,6 @@ __device__ __forceinline__ void acc_ld(uint32_t acc, const Role &ro, int c0, flo
   for (int i = 0; i < N; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// H = SiLU(acc + b) for this thread's 64 columns, into a [128][128] buffer, 32
-// columns at a time (80 registers hold three teams of 256 threads an SM).  The
-// biases are read four to a load: with one each, they were half of the
-// epilogue's instructions to the shared-memory and special-function queue.
-__device__ __forceinline__ void epi_silu(uint32_t acc, const Role &ro, const float *hb,
-                                         uint8_t *hout) {
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int c0 = ro.part * 64 + 32 * h;
-    float v[32];
-    acc_ld<32>(acc, ro, c0, v);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float4 b = *reinterpret_cast<const float4 *>(hb + c0 + 4 * i);
-      v[4 * i] = silu_h(fmaf(0.5f, v[4 * i], b.x));
-      v[4 * i + 1] = silu_h(fmaf(0.5f, v[4 * i + 1], b.y));
-      v[4 * i + 2] = silu_h(fmaf(0.5f, v[4 * i + 2], b.z));
-      v[4 * i + 3] = silu_h(fmaf(0.5f, v[4 * i + 3], b.w));
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) st_row8(hout, ro.row, c0 + 8 * k, kH, v + 8 * k);
-  }
-}
-
 // Normalised features of one sample into the X tile (zero padding to 16).
 __device__ __forceinline__ void put_raw(uint8_t *sx, int row, const float *raw, bool live,
                                         const MlpTileArgs &ta) {
@@ -294,55 +270,67 @@ __device__ __forceinline__ void load_weights(uint8_t *sm, float *bias,
 }
 
 // ---------------------------------------------------------------------------
-// inference: y[n][2] from x[n][5]; three teams of 256 threads per CTA
+// inference: y[n][2] from x[n][5]; six teams of 128 threads per CTA
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kFwdTeams * kTeam, 1)
+__global__ void __launch_bounds__(kFwdTeams * kFwdTeam, 1)
     k_mlp_forward(const uint8_t *__restrict__ wimg, const float *__restrict__ params,
                   const float *__restrict__ x, int nsamp, MlpTileArgs ta, float *__restrict__ y,
                   int *err) {
+  constexpr int T = kFwdTile;
   extern __shared__ __align__(1024) uint8_t sm[];
   __shared__ uint64_t bars[kFwdTeams];
   __shared__ uint32_t tslot;
-  const int tid = threadIdx.x, team_id = tid / kTeam, t = tid % kTeam;
-  if (tid < 32) tc::tmem_alloc(&tslot, 512);  // 128 columns a team, a power of two
+  const int tid = threadIdx.x, team_id = tid / kFwdTeam, t = tid % kFwdTeam;
+  if (tid < 32) tc::tmem_alloc(&tslot, 512);  // T columns a team, a power of two
   if (tid == 0) {
     for (int i = 0; i < kFwdTeams; ++i) tc::mbar_init(&bars[i], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   float *bias = reinterpret_cast<float *>(sm + fBias);
-  load_weights<kFwdTeams * kTeam>(sm, bias, wimg, params);
+  load_weights<kFwdTeams * kFwdTeam>(sm, bias, wimg, params);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const Role ro(t);
-  uint8_t *sx = sm + fTeam0 + team_id * (kXBytes + kHBytes), *sh = sx + kXBytes;
-  const uint32_t acc = tslot + 128 * team_id;
-  Gemm g{Team{1u + team_id, kTeam}, &bars[team_id], 0u, err, t == 0, false};
-  const int ntiles = (nsamp + kTile - 1) / kTile;
-  // this thread's inputs of its next tile, loaded one tile ahead
+  uint8_t *sx = sm + fTeam0 + team_id * kFwdTeamBytes, *sh = sx + T * kIn * 2;
+  const uint32_t acc = tslot + T * team_id;
+  Gemm g{Team{1u + team_id, kFwdTeam}, &bars[team_id], 0u, err, t == 0, false};
+  // H^T = SiLU(acc + b) of this thread's feature, 32 samples at a time
+  auto epilogue = [&](float hb) {
+#pragma unroll
+    for (int c = 0; c < T; c += 32) {
+      float v[32];
+      acc_ld<32>(acc, ro, c, v);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = silu_h(fmaf(0.5f, v[i], hb));
+#pragma unroll
+      for (int k = 0; k < 32; k += 8) st_row8(sh, ro.row, c + k, T, v + k);
+    }
+  };
+  const int ntiles = (nsamp + T - 1) / T, ahead = kFwdTeams * gridDim.x * T;
+  // this thread's sample of its team's next tile, loaded one tile ahead
+  const bool sample = ro.row < T;
+  int tile = team_id * gridDim.x + blockIdx.x;
   float raw[5];
-  {
-    const int s0 = (kFwdTeams * blockIdx.x + team_id) * kTile + ro.row;
-    load_raw(x, s0, ro.part == 0 && s0 < nsamp, raw);
-  }
-  for (int tile = kFwdTeams * blockIdx.x + team_id; tile < ntiles;
-       tile += kFwdTeams * gridDim.x) {
-    const int s = tile * kTile + ro.row;
-    const bool live = s < nsamp;
-    if (ro.part == 0) {
+  load_raw(x, tile * T + ro.row, sample && tile < ntiles && tile * T + ro.row < nsamp, raw);
+  for (; tile < ntiles; tile += kFwdTeams * gridDim.x) {
+    const int s = tile * T + ro.row;
+    const bool live = sample && s < nsamp;
+    if (sample) {
       put_raw(sx, ro.row, raw, live, ta);
-      const int ahead = kFwdTeams * gridDim.x * kTile;
       load_raw(x, s + ahead, s < nsamp - ahead, raw);
     }
-    if (!g.run(acc, sx, kIn, 0, sm + sW1, kIn, 0, kH, kIn)) break;
-    epi_silu(acc, ro, bias, sh);
+    if (!g.run(acc, sm + sW1, kIn, 0, sx, kIn, 0, T, kIn)) break;
+    epilogue(bias[ro.row]);
     bool ok = true;
     for (int l = 1; l < 4 && ok; ++l) {
-      ok = g.run(acc, sh, kH, 0, sm + sW2 + (l - 1) * kH * kH * 2, kH, 0, kH, kH);
-      if (ok) epi_silu(acc, ro, bias + l * kH, sh);
+      ok = g.run(acc, sm + sW2 + (l - 1) * kH * kH * 2, kH, 0, sh, T, 1, T, kH);
+      if (ok) epilogue(bias[l * kH + ro.row]);
     }
-    if (!ok || !g.run(acc, sh, kH, 0, sm + sW5, kH, 0, kOut, kH)) break;
-    if (ro.part == 0) {
+    // lanes are samples here; the upper 64 come from what lies behind H^T (at
+    // most 1 KB past it) and are not used
+    if (!ok || !g.run(acc, sh, T, 1, sm + sW5, kH, 0, kOut, kH)) break;
+    if (sample) {
       float v[16];
       acc_ld<16>(acc, ro, 0, v);
       if (live && !g.failed) {
@@ -999,10 +987,11 @@ extern "C" int qpsdm_mlp_forward(qpsdm_mlp *h, const float *d_x, int n, float *d
                                  void *stream) {
   if (!h || !d_x || !d_y || n <= 0) return QPSDM_EINVAL;
   cudaSetDevice(h->device);
-  const int ctas = ((n + kTile - 1) / kTile + kFwdTeams - 1) / kFwdTeams;
-  const int grid = ctas < h->nsm ? ctas : h->nsm;
-  k_mlp_forward<<<grid, kFwdTeams * kTeam, kFwdSmem, (cudaStream_t)stream>>>(h->wimg, h->p, d_x, n,
-                                                                     h->ta, d_y, h->err);
+  // a tile to an SM before a second team has one
+  const int ntiles = (n + kFwdTile - 1) / kFwdTile;
+  const int grid = ntiles < h->nsm ? ntiles : h->nsm;
+  k_mlp_forward<<<grid, kFwdTeams * kFwdTeam, kFwdSmem, (cudaStream_t)stream>>>(
+      h->wimg, h->p, d_x, n, h->ta, d_y, h->err);
   return cudaGetLastError() == cudaSuccess ? QPSDM_OK : QPSDM_ECUDA;
 }
 
