@@ -1164,7 +1164,7 @@ __global__ void __launch_bounds__(256)
     const float t = __fadd_rn(ts, tg);
     const float ft = __fmul_rn(t, inv_dt1);
     const int it1 = (int)ft;
-    if (!(it1 > 0 && it1 + 1 < a.nt)) return false;
+    if (!(it1 > 0 && it1 < a.nt - 1)) return false;  // (it1 is INT_MAX past its range)
     ++cimg;
     const float wt = __fsub_rn(ft, (float)it1);
     const float fb = fminf(fmaxf(__fmul_rn(__fadd_rn(qs, qg), inv_dts), 0.0f),
@@ -1626,7 +1626,7 @@ __global__ void __launch_bounds__(TZ *TX, MB)
               const float t = ts + tg;
               const float ft = t * inv_dt1;
               const int it1 = (int)ft;
-              if (!(it1 > 0 && it1 + 1 < a.nt)) continue;
+              if (!(it1 > 0 && it1 < a.nt - 1)) continue;  // (it1: INT_MAX past its range)
               const float fb = fminf(fmaxf(tq.y + qg, 0.0f), (float)(a.nbins - 1));
               const int b0 = min((int)fb, a.nbins - 2);
               fwt[u] = ft - (float)it1;
