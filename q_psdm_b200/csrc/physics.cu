@@ -2119,7 +2119,7 @@ __global__ void __launch_bounds__(TZ *TX / 2, MB)
               const float4 F2 = m[2 * splane], F3 = m[3 * splane];
               const unsigned long long t = f2_add(f2_pack(F2.x, F2.y), tg);
               const unsigned long long ft = f2_mul(t, f2_dup(inv_dt1));
-              // floor in the low bits (ft < 0 and NaN fail the window test)
+              // floor in the low bits (ft < 0, ft past 2^23 and NaN fail the window test)
               const unsigned long long mt = f2_add_rz(ft, two23);
               fwt[u] = f2_sub(ft, f2_sub(mt, two23));
               const float2 fbr = f2_unpack(f2_add(f2_pack(F2.z, F2.w), qg));
@@ -2156,7 +2156,12 @@ __global__ void __launch_bounds__(TZ *TX / 2, MB)
               const float2 fv = f2_unpack(
                   f2_mul(f2_mul(wt, f2_fma(r, r, f2_dup(1.0f))),
                          f2_mul(f2_mul(f2_dup(__int_as_float(rec[u].w)), uz), inv)));
+              // a lane that is off adds 0 times an interpolation of zeros: its factor
+              // and, since t may be infinite or NaN there, its time weight are 0
+              // (0.2 % of the kernel; choosing between the old and the new sum took 6 %)
               fac[u] = f2_pack(on[u][0] ? fv.x : 0.0f, on[u][1] ? fv.y : 0.0f);
+              const float2 wv = f2_unpack(fwt[u]);
+              fwt[u] = f2_pack(on[u][0] ? wv.x : 0.0f, on[u][1] ? wv.y : 0.0f);
               cimg += on[u][0];
               cimg += on[u][1];
             }

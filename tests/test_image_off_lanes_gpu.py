@@ -1,0 +1,53 @@
+"""The fast batched form computes a pair of depths, and two members, together:
+what it computes for a point or a member that takes no part must not reach the
+image.  Every fast variant against the plain form, FP32 panels: 2e-5 of the
+image peak (the bound the batched form is held to point by point), equal
+point-trace counts, every value finite."""
+import numpy as np
+import pytest
+
+from q_psdm_b200 import tables
+from tests.physics_case import make_case, records
+from tests.test_window_overflow_gpu import BAD, image, marked_case
+
+pytestmark = pytest.mark.gpu
+FAST = list(range(14, 28))
+
+
+def _check(c, rec, variant, kahan):
+    plain, s0 = image(c, rec, form=0, kahan=kahan)
+    img, s1 = image(c, rec, form=1, kahan=kahan, variant=variant)
+    amp = np.abs(plain).max()
+    assert np.isfinite(plain).all() and amp > 0
+    assert s1["point_traces"] == s0["point_traces"]
+    assert np.isfinite(img).all()
+    assert np.abs(img - plain).max() <= 2e-5 * amp
+
+
+@pytest.mark.parametrize("kahan", [0, 1])
+@pytest.mark.parametrize("variant", FAST)
+@pytest.mark.parametrize("shots", [(5, 9), (9, 5)])
+def test_first_source_off_the_tables(cuda, shots, variant, kahan):
+    """Two shots 260 m apart on tables that reach 320 m: some tiles' tables
+    cover the batch's second source and not its first."""
+    c = make_case(shots=shots, rstep=2)
+    sv = c["sv"]
+    c["tab"] = tables.linear_gradient_tables(sv, fci=sv.fci, nxi=sv.nxi, dxi=sv.dxi,
+                                             zmax=(sv.nzi - 1) * sv.dzi, sub=4, nxi1=16,
+                                             half_x=320.0, half_y=500.0)
+    _check(c, records(c), variant, kahan)
+
+
+@pytest.mark.parametrize("variant,kahan", [(v, 0) for v in FAST] + [(15, 1), (20, 1), (27, 1)])
+@pytest.mark.parametrize("bad", list(BAD))
+def test_nodes_past_the_window(cuda, bad, variant, kahan):
+    c = marked_case(BAD[bad])
+    _check(c, records(c), variant, kahan)
+
+
+@pytest.mark.parametrize("bad", list(BAD))
+@pytest.mark.parametrize("table,ntr", [("qqq", 512), ("ttt", 60)])
+def test_nodes_past_the_bins_and_unsplit(cuda, bad, table, ntr):
+    c = marked_case(BAD[bad], table)
+    rec = records(c)
+    _check(c, rec[np.linspace(0, rec.shape[0] - 1, ntr).astype(int)], 26, 0)
