@@ -60,7 +60,7 @@ __device__ __forceinline__ float lin_grad_time(float r, float z, float v0, float
 // sweep's list (a node's update depends on its six neighbours alone, so a
 // node left out would have kept its value).  Lists, the sweep a block was last
 // listed for and the marks of blocks with start nodes (the only ones that sweep
-// 0 visits) live in the t* output until it is written.
+// 0 visits; for t*, then, of blocks visited) live in the t* output until it is written.
 constexpr int kEx = 16, kEy = 8, kEz = 4, kEikThreads = kEx * kEy * kEz / 2;
 
 // n / d for n < 2^31 as a multiply-high and a shift: with 2^(l-1) < d <= 2^l,
@@ -85,7 +85,7 @@ struct EikBlocks {
   int nbx, nby, nbz, nblk;  // blocks per axis, blocks of all sources
   EikDiv row, plane, grid;  // by nbx, nbx nby, nbx nby nbz
   int *list0, *list1;       // blocks of even and odd sweeps, [nblk] each
-  int *listed, *seed;       // sweep a block was last listed for; holds start nodes
+  int *listed, *seed;       // sweep a block was last listed for; holds start nodes / visited
   unsigned *count;          // list lengths of three consecutive sweeps, in turn
 };
 
@@ -291,7 +291,9 @@ __global__ void __launch_bounds__(kEikThreads)
 // it changes.  In sweep 0 the blocks that hold start nodes, and after it what
 // they reach: t* at a node depends on nodes of smaller T only, so the values
 // settle outwards from the source, most blocks in a few visits, and a block is
-// listed only for a changed neighbour of smaller T.  256 sweeps over every
+// listed only for a neighbour of smaller T that has changed, or whose block is
+// visited for the first time: a value that stays at its initial 0 (no attenuation
+// so far) must be carried on too.  256 sweeps over every
 // node took 95 ms for the 28 M nodes of 32 sources; so 6.9 ms; 4.7 ms with the
 // traveltimes of the neighbours from shared memory, a halo of the facing nodes
 // only and the seed marks (a visit's preparation, not its FP64 updates, is most
@@ -327,6 +329,7 @@ __global__ void __launch_bounds__(kTsThreads)
     bool on = e.x0 + lx < g.nx && e.y0 + ly < g.ny && e.z0 + lz < g.nz;
     const size_t i = e.base + lz * sxy + (size_t)ly * g.nx + lx;
     const bool start = on && F[i] < 0.0f;
+    const bool first = sweep == 0 || !B.seed[blk];  // seed: blocks visited, from here on
     if (threadIdx.x == 0) s_faces = 0;
     // the block and the nodes facing it
     const float ti = on ? T[i] : kInf;
@@ -383,10 +386,11 @@ __global__ void __launch_bounds__(kTsThreads)
     }
     if (on && __double_as_longlong(val) != __double_as_longlong(old))
       TS[i] = val;
-    else if (sweep > 0)
-      faces = 0;  // (start nodes may fill the block: sweep 0 lists what is downwind of them)
+    else if (!first)
+      faces = 0;
     if (more) faces |= 1u;  // settled, unless the loop ran out
     if (faces) atomicOr(&s_faces, faces);
+    if (threadIdx.x == 0) B.seed[blk] = 1;
     __syncthreads();
     eik_mark(B, blk, e, s_faces, sweep);
     __syncthreads();

@@ -29,13 +29,16 @@ def _check(c, rec, variant, kahan):
 @pytest.mark.parametrize("shots", [(5, 9), (9, 5)])
 def test_first_source_off_the_tables(cuda, shots, variant, kahan):
     """Two shots 260 m apart on tables that reach 320 m: some tiles' tables
-    cover the batch's second source and not its first."""
+    cover the batch's second source and not its first.  Of the gathers' traces
+    a random 300, so that the parts of the members end anywhere in the spread."""
     c = make_case(shots=shots, rstep=2)
     sv = c["sv"]
     c["tab"] = tables.linear_gradient_tables(sv, fci=sv.fci, nxi=sv.nxi, dxi=sv.dxi,
                                              zmax=(sv.nzi - 1) * sv.dzi, sub=4, nxi1=16,
                                              half_x=320.0, half_y=500.0)
-    _check(c, records(c), variant, kahan)
+    rec = records(c)
+    rng = np.random.default_rng(variant)
+    _check(c, rec[np.sort(rng.permutation(rec.shape[0])[:300])], variant, kahan)
 
 
 @pytest.mark.parametrize("variant,kahan", [(v, 0) for v in FAST] + [(15, 1), (20, 1), (27, 1)])
