@@ -358,16 +358,20 @@ static int check_tables(const qpsdm_line_params &l, std::string *err) {
 // (the reference layout, depth fastest) re-laid out as [nzi1][nxi1] (cdp
 // fastest), so that image points of neighbouring cdps, which a warp of the
 // batched kernel holds, read neighbouring table words.  Out of place:
-// descriptors may share a block.
+// descriptors may share a block.  gridDim.y CTAs share the ncell cells.
 __global__ void k_tab_xfast(const float *__restrict__ in, float *__restrict__ out,
-                            const qpsdm_ttt_desc *__restrict__ desc, int nxi1, int nzi1) {
-  const qpsdm_ttt_desc d = desc[blockIdx.y];
-  const int nplanes = (int)d.nys * d.nxs, plane = nxi1 * nzi1;
-  for (int pl = blockIdx.x; pl < nplanes; pl += gridDim.x) {
-    const int64_t base = d.idx + (int64_t)pl * plane;
-    for (int e = threadIdx.x; e < plane; e += blockDim.x) {
-      const int ixl = e / nzi1, izl = e - ixl * nzi1;
-      out[base + izl * nxi1 + ixl] = in[base + e];
+                            const qpsdm_ttt_desc *__restrict__ desc, int ncell, int nxi1,
+                            int nzi1) {
+  const int plane = nxi1 * nzi1;
+  for (int c = blockIdx.y; c < ncell; c += gridDim.y) {
+    const qpsdm_ttt_desc d = desc[c];
+    const int nplanes = (int)d.nys * d.nxs;
+    for (int pl = blockIdx.x; pl < nplanes; pl += gridDim.x) {
+      const int64_t base = d.idx + (int64_t)pl * plane;
+      for (int e = threadIdx.x; e < plane; e += blockDim.x) {
+        const int ixl = e / nzi1, izl = e - ixl * nzi1;
+        out[base + izl * nxi1 + ixl] = in[base + e];
+      }
     }
   }
 }
@@ -375,28 +379,30 @@ __global__ void k_tab_xfast(const float *__restrict__ in, float *__restrict__ ou
 // Two tables with identical descriptors as one array of (t, t*) of a node and
 // (t, t*) of the node below it, cdp fastest (batched form) or in the tables' own
 // order: a receiver's lookup at both depth nodes of a point is four 16-byte
-// loads instead of eight 8-byte or sixteen 4-byte ones.  Below a cell's last node comes the first node of the cell under it
-// (on the same surface grid; else, and below the deepest cell, the node
-// itself, whose weight is zero).
+// loads instead of eight 8-byte or sixteen 4-byte ones.  Below a cell's last
+// node comes the first node of the cell under it (on the same surface grid;
+// else, and below the deepest cell, the node itself, whose weight is zero).
 __global__ void k_tab_quads(const float *__restrict__ t, const float *__restrict__ q,
                             float4 *__restrict__ out, const qpsdm_ttt_desc *__restrict__ desc,
-                            int nzg, int nxi1, int nzi1, int xfast) {
-  const int c = blockIdx.y;
-  const qpsdm_ttt_desc d = desc[c];
-  const int nplanes = (int)d.nys * d.nxs, plane = nxi1 * nzi1;
-  int64_t under = -1;
-  if ((c + 1) % nzg != 0) {
-    const qpsdm_ttt_desc e = desc[c + 1];
-    if (e.nys == d.nys && e.nxs == d.nxs && e.dys == d.dys && e.dxs == d.dxs) under = e.idx;
-  }
-  for (int pl = blockIdx.x; pl < nplanes; pl += gridDim.x) {
-    const int64_t base = d.idx + (int64_t)pl * plane, ub = under + (int64_t)pl * plane;
-    for (int o = threadIdx.x; o < plane; o += blockDim.x) {
-      const int izl = xfast ? o / nxi1 : o % nzi1;
-      const int ixl = xfast ? o - izl * nxi1 : o / nzi1;
-      const int64_t i = base + ixl * nzi1 + izl;
-      const int64_t j = izl + 1 < nzi1 ? i + 1 : under >= 0 ? ub + ixl * nzi1 : i;
-      out[base + o] = make_float4(t[i], q[i], t[j], q[j]);
+                            int ncell, int nzg, int nxi1, int nzi1, int xfast) {
+  const int plane = nxi1 * nzi1;
+  for (int c = blockIdx.y; c < ncell; c += gridDim.y) {
+    const qpsdm_ttt_desc d = desc[c];
+    const int nplanes = (int)d.nys * d.nxs;
+    int64_t under = -1;
+    if ((c + 1) % nzg != 0) {
+      const qpsdm_ttt_desc e = desc[c + 1];
+      if (e.nys == d.nys && e.nxs == d.nxs && e.dys == d.dys && e.dxs == d.dxs) under = e.idx;
+    }
+    for (int pl = blockIdx.x; pl < nplanes; pl += gridDim.x) {
+      const int64_t base = d.idx + (int64_t)pl * plane, ub = under + (int64_t)pl * plane;
+      for (int o = threadIdx.x; o < plane; o += blockDim.x) {
+        const int izl = xfast ? o / nxi1 : o % nzi1;
+        const int ixl = xfast ? o - izl * nxi1 : o / nzi1;
+        const int64_t i = base + ixl * nzi1 + izl;
+        const int64_t j = izl + 1 < nzi1 ? i + 1 : under >= 0 ? ub + ixl * nzi1 : i;
+        out[base + o] = make_float4(t[i], q[i], t[j], q[j]);
+      }
     }
   }
 }
@@ -467,7 +473,8 @@ int physics_set_lines(PhysicsState *s, const qpsdm_static_params &p,
       cudaMemcpyAsync(t.qqq, l.qqq, sizeof(float) * l.qqq_len, cudaMemcpyDefault, st);
     }
     if (!t.paired && !batched) continue;
-    const dim3 g(256, (unsigned)ncell);
+    const int nc = (int)ncell;  // positive ints nxg, nzg; cells past a grid's 65,535 in turn
+    const dim3 g(256, (unsigned)std::min(nc, 65535));
     const float *src[2] = {on_device(l.ttt, dev), on_device(l.qqq, dev)};
     if (!src[0] || !src[1]) {
       if (!grow_dev(&s->d_tab_tmp, &s->tab_tmp_cap, (size_t)(l.ttt_len + l.qqq_len))) {
@@ -489,14 +496,15 @@ int physics_set_lines(PhysicsState *s, const qpsdm_static_params &p,
         if (err) *err = "paired table allocation failed";
         return QPSDM_ENOMEM;
       }
-      k_tab_quads<<<g, 256, 0, st>>>(src[0], src[1], t.tq, t.dt, l.nzg, l.nxi1, l.nzi1, batched);
+      k_tab_quads<<<g, 256, 0, st>>>(src[0], src[1], t.tq, t.dt, nc, l.nzg, l.nxi1, l.nzi1,
+                                   batched);
     }
     if (single && batched) {
-      k_tab_xfast<<<g, 256, 0, st>>>(src[0], t.ttt, t.dt, l.nxi1, l.nzi1);
-      k_tab_xfast<<<g, 256, 0, st>>>(src[1], t.qqq, t.dq, l.nxi1, l.nzi1);
+      k_tab_xfast<<<g, 256, 0, st>>>(src[0], t.ttt, t.dt, nc, l.nxi1, l.nzi1);
+      k_tab_xfast<<<g, 256, 0, st>>>(src[1], t.qqq, t.dq, nc, l.nxi1, l.nzi1);
     }
   }
-  if (cudaStreamSynchronize(st) != cudaSuccess) {
+  if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) {
     if (err) *err = "table upload failed";
     return QPSDM_ECUDA;
   }
