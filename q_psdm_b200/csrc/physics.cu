@@ -407,17 +407,31 @@ __global__ void k_tab_quads(const float *__restrict__ t, const float *__restrict
   }
 }
 
-// Whether no two cells of a line's traveltime tables share data: with more than
-// one depth cell, a shared block may have different cells under it.
-static bool disjoint_blocks(const qpsdm_line_params &l) {
-  std::vector<std::pair<int64_t, int64_t>> b((size_t)l.nxg * l.nzg);
+// Whether one quad per table entry serves every cell of a line that reads the
+// entry: blocks that overlap have their planes at the same places, and the node
+// under their last one equally far on (cells that share a v(z) table column by
+// column do; blocks shared by cells of different depths do not).
+static bool quads_fit(const qpsdm_line_params &l) {
+  struct Block {
+    int64_t lo, hi, under;
+  };
+  const int64_t plane = (int64_t)l.nxi1 * l.nzi1;
+  std::vector<Block> b((size_t)l.nxg * l.nzg);
   for (size_t c = 0; c < b.size(); ++c) {
     const qpsdm_ttt_desc &d = l.ttt_desc[c];
-    b[c] = {d.idx, d.idx + (int64_t)d.nys * d.nxs * l.nxi1 * l.nzi1};
+    b[c] = {d.idx, d.idx + (int64_t)d.nys * d.nxs * plane, INT64_MIN};
+    if ((c + 1) % l.nzg != 0) {
+      const qpsdm_ttt_desc &e = l.ttt_desc[c + 1];
+      if (e.nys == d.nys && e.nxs == d.nxs && e.dys == d.dys && e.dxs == d.dxs)
+        b[c].under = e.idx - d.idx;
+    }
   }
-  std::sort(b.begin(), b.end());
-  for (size_t c = 1; c < b.size(); ++c)
-    if (b[c].first < b[c - 1].second) return false;
+  std::sort(b.begin(), b.end(), [](const Block &x, const Block &y) { return x.lo < y.lo; });
+  Block far = b[0];  // of the blocks so far, the one that ends last
+  for (const Block &x : b) {
+    if (x.lo < far.hi && ((x.lo - far.lo) % plane != 0 || x.under != far.under)) return false;
+    if (x.hi > far.hi) far = x;
+  }
   return true;
 }
 
@@ -457,7 +471,7 @@ int physics_set_lines(PhysicsState *s, const qpsdm_static_params &p,
     // of a node are read together
     t.paired = l.ttt_len == l.qqq_len &&
                std::memcmp(l.ttt_desc, l.qqq_desc, sizeof(qpsdm_ttt_desc) * ncell) == 0 &&
-               (l.nzg == 1 || disjoint_blocks(l));
+               quads_fit(l);
     // paired tables on one surface grid need no table of their own
     const bool single = !(t.paired && t.one_grid), batched = s->form == QPSDM_FORM_BATCHED;
     if (!grow_dev(&t.dt, &t.dt_cap, ncell) || !grow_dev(&t.dq, &t.dq_cap, ncell) ||
