@@ -71,6 +71,7 @@ struct GroupSet {
 // most, and the most sums that the parts of an image leave (32 MB per set).
 constexpr int kMaxSplit = 32, kSplitChunk = 256;
 constexpr size_t kSplitSums = 1 << 23;
+constexpr size_t kTabTmpKeep = 1 << 25;  // floats of table staging the plain form keeps
 
 struct PhysicsState {
   int nfft = 0, nffti = 0, nbins = 0, max_batch = 0, dtype = 0;
@@ -96,7 +97,7 @@ struct PhysicsState {
     bool one_grid = false;  // every cell has the same surface grid
   };
   std::vector<LineTab> tabs;  // one per line of the brick
-  float *d_tab_tmp = nullptr;  // batched form: table upload before the re-layout
+  float *d_tab_tmp = nullptr;  // a table from the host before its re-layout
   size_t tab_tmp_cap = 0;
   int ntabs = 0;
   int *d_any = nullptr;       // [max_batch] accepted by any line of the brick
@@ -322,7 +323,10 @@ static bool grow_dev(T **p, size_t *cap, size_t need) {
   cudaFree(*p);
   *p = nullptr;
   *cap = 0;
-  if (cudaMalloc((void **)p, sizeof(T) * (need ? need : 1)) != cudaSuccess) return false;
+  if (cudaMalloc((void **)p, sizeof(T) * (need ? need : 1)) != cudaSuccess) {
+    cudaGetLastError();  // told by the result: the caller may have another way
+    return false;
+  }
   *cap = need;
   return true;
 }
@@ -382,6 +386,7 @@ __global__ void k_tab_xfast(const float *__restrict__ in, float *__restrict__ ou
 // loads instead of eight 8-byte or sixteen 4-byte ones.  Below a cell's last
 // node comes the first node of the cell under it (on the same surface grid;
 // else, and below the deepest cell, the node itself, whose weight is zero).
+// With one table null, the other's halves of the quads alone are written.
 __global__ void k_tab_quads(const float *__restrict__ t, const float *__restrict__ q,
                             float4 *__restrict__ out, const qpsdm_ttt_desc *__restrict__ desc,
                             int ncell, int nzg, int nxi1, int nzi1, int xfast) {
@@ -401,7 +406,13 @@ __global__ void k_tab_quads(const float *__restrict__ t, const float *__restrict
         const int ixl = xfast ? o - izl * nxi1 : o / nzi1;
         const int64_t i = base + ixl * nzi1 + izl;
         const int64_t j = izl + 1 < nzi1 ? i + 1 : under >= 0 ? ub + ixl * nzi1 : i;
-        out[base + o] = make_float4(t[i], q[i], t[j], q[j]);
+        float4 &w = out[base + o];
+        if (t && q)
+          w = make_float4(t[i], q[i], t[j], q[j]);
+        else if (t)
+          w.x = t[i], w.z = t[j];
+        else
+          w.y = q[i], w.w = q[j];
       }
     }
   }
@@ -435,27 +446,20 @@ static bool quads_fit(const qpsdm_line_params &l) {
   return true;
 }
 
-// Table data may be host memory or memory of the engine's device; descriptors
-// are host memory.
-int physics_set_lines(PhysicsState *s, const qpsdm_static_params &p,
-                      const qpsdm_line_params *lines, int nlines, cudaStream_t st,
-                      std::string *err) {
-  (void)p;
-  for (int il = 0; il < nlines; ++il) {
-    int rc = check_tables(lines[il], err);
-    if (rc) return rc;
-  }
-  if ((int)s->tabs.size() < nlines) s->tabs.resize(nlines);
+// Tables of a brick's lines; (t, t*) quads where `pair` and the tables allow it.
+static int upload_lines(PhysicsState *s, const qpsdm_line_params *lines, int nlines, bool pair,
+                        cudaStream_t st) {
   int dev = 0;
   cudaGetDevice(&dev);
   // data already in this device's memory is read in place
-  auto on_device = [](const float *p, int d) -> const float * {
+  auto on_device = [dev](const float *p) {
     cudaPointerAttributes at;
     const bool yes = cudaPointerGetAttributes(&at, p) == cudaSuccess &&
-                     at.type == cudaMemoryTypeDevice && at.device == d;
+                     at.type == cudaMemoryTypeDevice && at.device == dev;
     cudaGetLastError();  // a pageable pointer may leave an error behind
-    return yes ? p : nullptr;
+    return yes;
   };
+  const bool batched = s->form == QPSDM_FORM_BATCHED;
   for (int il = 0; il < nlines; ++il) {
     const qpsdm_line_params &l = lines[il];
     PhysicsState::LineTab &t = s->tabs[il];
@@ -469,59 +473,88 @@ int physics_set_lines(PhysicsState *s, const qpsdm_static_params &p,
                    (int64_t)l.ttt_desc[c].nxs * l.ttt_desc[c].nys * l.nxi1 * l.nzi1 < (1ll << 30);
     // identical descriptors (the reference writes both tables alike): t and t*
     // of a node are read together
-    t.paired = l.ttt_len == l.qqq_len &&
+    t.paired = pair && l.ttt_len == l.qqq_len &&
                std::memcmp(l.ttt_desc, l.qqq_desc, sizeof(qpsdm_ttt_desc) * ncell) == 0 &&
                quads_fit(l);
     // paired tables on one surface grid need no table of their own
-    const bool single = !(t.paired && t.one_grid), batched = s->form == QPSDM_FORM_BATCHED;
+    const bool single = !(t.paired && t.one_grid);
     if (!grow_dev(&t.dt, &t.dt_cap, ncell) || !grow_dev(&t.dq, &t.dq_cap, ncell) ||
         (single && (!grow_dev(&t.ttt, &t.ttt_cap, (size_t)l.ttt_len) ||
-                    !grow_dev(&t.qqq, &t.qqq_cap, (size_t)l.qqq_len)))) {
-      if (err) *err = "table allocation failed";
+                    !grow_dev(&t.qqq, &t.qqq_cap, (size_t)l.qqq_len))) ||
+        (t.paired && !grow_dev(&t.tq, &t.tq_cap, (size_t)l.ttt_len)))
       return QPSDM_ENOMEM;
-    }
     cudaMemcpyAsync(t.dt, l.ttt_desc, sizeof(qpsdm_ttt_desc) * ncell, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(t.dq, l.qqq_desc, sizeof(qpsdm_ttt_desc) * ncell, cudaMemcpyHostToDevice, st);
-    if (single && !batched) {
-      cudaMemcpyAsync(t.ttt, l.ttt, sizeof(float) * l.ttt_len, cudaMemcpyDefault, st);
-      cudaMemcpyAsync(t.qqq, l.qqq, sizeof(float) * l.qqq_len, cudaMemcpyDefault, st);
-    }
-    if (!t.paired && !batched) continue;
-    const int nc = (int)ncell;  // positive ints nxg, nzg; cells past a grid's 65,535 in turn
+    const int nc = (int)ncell;  // cells past a grid's 65,535 rows come in turn
     const dim3 g(256, (unsigned)std::min(nc, 65535));
-    const float *src[2] = {on_device(l.ttt, dev), on_device(l.qqq, dev)};
-    if (!src[0] || !src[1]) {
-      if (!grow_dev(&s->d_tab_tmp, &s->tab_tmp_cap, (size_t)(l.ttt_len + l.qqq_len))) {
-        if (err) *err = "table re-layout scratch allocation failed";
-        return QPSDM_ENOMEM;
+    // a table in host memory passes through the staging copy, one after the other
+    const bool both = on_device(l.ttt) && on_device(l.qqq);
+    for (int w = 0; w < 2; ++w) {
+      const float *src = w ? l.qqq : l.ttt;
+      const size_t len = (size_t)(w ? l.qqq_len : l.ttt_len);
+      float *own = w ? t.qqq : t.ttt;
+      const qpsdm_ttt_desc *d = w ? t.dq : t.dt;
+      if (single && !batched)
+        cudaMemcpyAsync(own, src, sizeof(float) * len, cudaMemcpyDefault, st);
+      if (!t.paired && !batched) continue;
+      if (!both && !on_device(src)) {
+        if (!grow_dev(&s->d_tab_tmp, &s->tab_tmp_cap, len)) return QPSDM_ENOMEM;
+        cudaMemcpyAsync(s->d_tab_tmp, src, sizeof(float) * len, cudaMemcpyDefault, st);
+        src = s->d_tab_tmp;
       }
-      if (!src[0]) {
-        cudaMemcpyAsync(s->d_tab_tmp, l.ttt, sizeof(float) * l.ttt_len, cudaMemcpyDefault, st);
-        src[0] = s->d_tab_tmp;
-      }
-      if (!src[1]) {
-        cudaMemcpyAsync(s->d_tab_tmp + l.ttt_len, l.qqq, sizeof(float) * l.qqq_len,
-                        cudaMemcpyDefault, st);
-        src[1] = s->d_tab_tmp + l.ttt_len;
-      }
+      if (t.paired && (!both || w == 0))
+        k_tab_quads<<<g, 256, 0, st>>>(w ? nullptr : src, both ? l.qqq : w ? src : nullptr, t.tq,
+                                       d, nc, l.nzg, l.nxi1, l.nzi1, batched);
+      if (single && batched) k_tab_xfast<<<g, 256, 0, st>>>(src, own, d, nc, l.nxi1, l.nzi1);
     }
-    if (t.paired) {
-      if (!grow_dev(&t.tq, &t.tq_cap, (size_t)l.ttt_len)) {
-        if (err) *err = "paired table allocation failed";
-        return QPSDM_ENOMEM;
-      }
-      k_tab_quads<<<g, 256, 0, st>>>(src[0], src[1], t.tq, t.dt, nc, l.nzg, l.nxi1, l.nzi1,
-                                   batched);
+  }
+  return QPSDM_OK;
+}
+
+template <typename T>
+static void free_dev(T **p, size_t *cap) {
+  cudaFree(*p);
+  *p = nullptr;
+  *cap = 0;
+}
+
+// Table data may be host memory or memory of the engine's device; descriptors
+// are host memory.  Quads take 16 bytes an entry (24 beside the float tables,
+// with several surface grids); where they do not fit the GPU, every line gets
+// float tables alone, 8 bytes.
+int physics_set_lines(PhysicsState *s, const qpsdm_static_params &p,
+                      const qpsdm_line_params *lines, int nlines, cudaStream_t st,
+                      std::string *err) {
+  (void)p;
+  for (int il = 0; il < nlines; ++il) {
+    int rc = check_tables(lines[il], err);
+    if (rc) return rc;
+  }
+  if ((int)s->tabs.size() < nlines) s->tabs.resize(nlines);
+  int rc = upload_lines(s, lines, nlines, true, st);
+  if (rc == QPSDM_ENOMEM) {
+    cudaStreamSynchronize(st);
+    for (PhysicsState::LineTab &t : s->tabs) {
+      free_dev(&t.ttt, &t.ttt_cap);
+      free_dev(&t.qqq, &t.qqq_cap);
+      free_dev(&t.tq, &t.tq_cap);
     }
-    if (single && batched) {
-      k_tab_xfast<<<g, 256, 0, st>>>(src[0], t.ttt, t.dt, nc, l.nxi1, l.nzi1);
-      k_tab_xfast<<<g, 256, 0, st>>>(src[1], t.qqq, t.dq, nc, l.nxi1, l.nzi1);
-    }
+    free_dev(&s->d_tab_tmp, &s->tab_tmp_cap);
+    s->ntabs = 0;
+    rc = upload_lines(s, lines, nlines, false, st);
+  }
+  if (rc) {
+    cudaStreamSynchronize(st);
+    if (err) *err = "table allocation failed";
+    return rc;
   }
   if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) {
     if (err) *err = "table upload failed";
     return QPSDM_ECUDA;
   }
+  // the plain form's staging copy: a small one is kept for the next lines
+  if (s->form == QPSDM_FORM_PLAIN && s->tab_tmp_cap > kTabTmpKeep)
+    free_dev(&s->d_tab_tmp, &s->tab_tmp_cap);
   s->ntabs = nlines;
   return QPSDM_OK;
 }
