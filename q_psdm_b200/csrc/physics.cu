@@ -68,7 +68,8 @@ struct GroupSet {
   void *d_cub = nullptr;
 };
 // Most parts a tile's members are split into, members of a part's chunks at
-// most, and the most sums that the parts of an image leave (32 MB per set).
+// most, and the most sums that the parts of an image leave (32 MB per set, 64
+// with compensated sums).
 constexpr int kMaxSplit = 32, kSplitChunk = 256;
 constexpr size_t kSplitSums = 1 << 23;
 constexpr size_t kTabTmpKeep = 1 << 25;  // floats of table staging the plain form keeps
@@ -118,6 +119,7 @@ struct PhysicsState {
   int *d_ndefer = nullptr;
   float *d_part = nullptr;
   size_t part_cap = 0;
+  size_t part_words = 1;                       // 2 with compensated sums
   int *d_nmem = nullptr;                       // accepted members of the current line's batch
   void *d_cub = nullptr;
   size_t cub_bytes = 0;
@@ -234,6 +236,7 @@ int physics_create(PhysicsState **out, const qpsdm_static_params &p, std::string
   s->dtstar = p.dtstar;
   s->max_batch = p.max_batch;
   s->dtype = p.panel_dtype;
+  s->part_words = p.kahan ? 2 : 1;
   std::vector<float2> f;
   std::vector<float> fmax;
   filter_table(p, p.nbins, p.dtstar, f, fmax, &s->kmax);
@@ -573,7 +576,8 @@ int physics_begin_offset(PhysicsState *s, const qpsdm_static_params &p,
     for (GroupSet &g : s->sets) {
       if (!grow_dev(&g.d_defer, &g.defer_cap, ntile) ||
           !grow_dev(&g.d_tile_ctr, &g.ctr_cap, 2 + ntile) ||
-          !grow_dev(&g.d_part, &g.part_cap, std::min(kMaxSplit * npt, kSplitSums))) {
+          !grow_dev(&g.d_part, &g.part_cap,
+                    std::min(kMaxSplit * npt, kSplitSums) * s->part_words)) {
         if (err) *err = "tile queue allocation failed";
         return QPSDM_ENOMEM;
       }
@@ -1362,22 +1366,39 @@ __device__ __forceinline__ bool last_part(int *done, int nsplit, int *s_flag) {
   __threadfence();
   return true;
 }
-// Adds a point's nsplit partial sums to the image in order.
+// A part's sum of a point, and its compensation behind it (compensated sums: a part
+// rounded to one float would lose what the compensation had kept).
+__device__ __forceinline__ void put_part(float *part, size_t nimg, int ipart, float acc, float cmp,
+                                         bool comp) {
+  if (comp) {
+    part[2 * ipart * nimg] = acc;
+    part[(2 * ipart + 1) * nimg] = cmp;
+  } else {
+    part[ipart * nimg] = acc;
+  }
+}
+// Adds a point's nsplit partial sums to the image in order.  Compensated: a sum
+// is s - c; parts are as large as the image, so the whole error of each addition
+// is taken (Knuth's two-sum), where a step of the compensated sum would round
+// the part minus c.
 __device__ __forceinline__ void add_parts(float *img, float *comp, const float *part, size_t nimg,
                                           int nsplit) {
-  float s = *img, c = comp ? *comp : 0.0f;
-  for (int i = 0; i < nsplit; ++i) {
-    const float v = __ldcg(part + i * nimg);
-    if (comp) {
-      const float y = v - c, tt = s + y;
-      c = (tt - s) - y;
-      s = tt;
-    } else {
-      s += v;
-    }
+  float s = *img;
+  if (!comp) {
+    for (int i = 0; i < nsplit; ++i) s += __ldcg(part + i * nimg);
+    *img = s;
+    return;
   }
-  *img = s;
-  if (comp) *comp = c;
+  float c = *comp;
+  for (int i = 0; i < nsplit; ++i) {
+    const float v = __ldcg(part + 2 * i * nimg), t = s + v, b = t - s;
+    const float e = (s - (t - b)) + (v - b);
+    c = (c - e) + __ldcg(part + (2 * i + 1) * nimg);
+    s = t;
+  }
+  const float t = s - c;
+  *img = t;
+  *comp = (t - s) + c;
 }
 
 // Batched imaging.  A persistent CTA takes image tiles of TZ depths x TX
@@ -1737,7 +1758,7 @@ __global__ void __launch_bounds__(TZ *TX, MB)
       continue;
     }
     const size_t nimg = (size_t)a.nxb * a.nzi;
-    if (live) part[ipart * nimg + o] = acc - cmp;
+    if (live) put_part(part + o, nimg, ipart, acc, cmp, comp);
     if (!last_part(tile_done + tile, nsplit, &s_tile)) continue;
     if (live) add_parts(img + o, comp ? comp + o : nullptr, part + o, nimg, nsplit);
   }
@@ -2270,7 +2291,8 @@ __global__ void __launch_bounds__(TZ *TX / 2, MB)
     const size_t nimg = (size_t)a.nxb * a.nzi;
 #pragma unroll
     for (int p = 0; p < 2; ++p)
-      if (live[p]) part[ipart * nimg + o + p] = (p ? av.y : av.x) - (p ? cv.y : cv.x);
+      if (live[p])
+        put_part(part + o + p, nimg, ipart, p ? av.y : av.x, p ? cv.y : cv.x, comp);
     if (!last_part(tile_done + tile, nsplit, &s_tile)) continue;
 #pragma unroll
     for (int p = 0; p < 2; ++p)
@@ -2380,7 +2402,7 @@ static_assert(kNumVariants <= 32, "tune_ms holds 32 timings");
 // is not split (1024 x 600: 2,432 tiles, 38.1 ms against 38.3 for eight lines).
 static int member_split(const PhysicsState *s, const PhysImageArgs &a, int ntiles, int ntr) {
   const int want = (32 * s->num_sms + ntiles - 1) / ntiles;
-  const size_t room = s->part_cap / ((size_t)a.nxb * a.nzi);
+  const size_t room = s->part_cap / (s->part_words * (size_t)a.nxb * a.nzi);
   return std::max(1, std::min(std::min(want, ntr / 64), std::min((int)room, kMaxSplit)));
 }
 
