@@ -575,15 +575,12 @@ int physics_begin_offset(PhysicsState *s, const qpsdm_static_params &p,
     const size_t npt = nxb * p.nzi, ntile = npt / 32 + nxb + p.nzi + 1;  // tiles: 32 points or more
     for (GroupSet &g : s->sets) {
       if (!grow_dev(&g.d_defer, &g.defer_cap, ntile) ||
-          !grow_dev(&g.d_tile_ctr, &g.ctr_cap, 2 + ntile) ||
-          !grow_dev(&g.d_part, &g.part_cap,
-                    std::min(kMaxSplit * npt, kSplitSums) * s->part_words)) {
+          !grow_dev(&g.d_tile_ctr, &g.ctr_cap, 2 + ntile)) {
         if (err) *err = "tile queue allocation failed";
         return QPSDM_ENOMEM;
       }
       g.d_ndefer = g.d_tile_ctr + 1;
     }
-    select_set(s, s->cur_set);
   }
   if (p.kahan) {
     const size_t n = (size_t)(o.ixend - o.ixstart) * p.nzi * nlines;
@@ -592,6 +589,13 @@ int physics_begin_offset(PhysicsState *s, const qpsdm_static_params &p,
       return QPSDM_ENOMEM;
     }
     cudaMemsetAsync(s->d_comp, 0, sizeof(float) * n, st);
+  }
+  if (s->form == QPSDM_FORM_BATCHED) {
+    // without room for the parts' sums no tile is split (member_split)
+    const size_t npt = (size_t)(o.ixend - o.ixstart) * p.nzi;
+    for (GroupSet &g : s->sets)
+      grow_dev(&g.d_part, &g.part_cap, std::min(kMaxSplit * npt, kSplitSums) * s->part_words);
+    select_set(s, s->cur_set);
   }
   return QPSDM_OK;
 }
