@@ -493,7 +493,9 @@ int qpsdm_eikonal_correct(const qpsdm_sur_line *ln, const qpsdm_ttt_desc *desc, 
  * max-accumulated into d_node_err (float per node, cells in descriptor
  * order, nodes [iys][ixs]; clear it first: calls for several lines give the
  * maximum over them).  desc: host descriptors; d_ttt: len floats (device).
- * Synchronises the stream. */
+ * Synchronises the stream.  This call and the next need about 117 MB of device
+ * memory besides their arguments, which the network's handle keeps for the
+ * calls to come until it is destroyed. */
 int qpsdm_surrogate_gate(qpsdm_mlp *net, const qpsdm_sur_line *ln, const qpsdm_ttt_desc *desc,
                          const float *d_ttt, int64_t len, float *d_node_err, void *stream);
 

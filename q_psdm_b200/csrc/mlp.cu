@@ -752,22 +752,24 @@ namespace qpsdm {
 
 // A device workspace of at least `bytes` for a call that ends with its work
 // done: the one the handle keeps if it is free and large enough, else a new
-// one.  mlp_put_workspace keeps it in the handle again (the larger of two
-// when calls overlapped) or frees it.
+// one, before which a kept one that is too small is given back.
+// mlp_put_workspace keeps it in the handle again (the larger of two when calls
+// overlapped) or frees it.
 void *mlp_take_workspace(qpsdm_mlp *h, size_t bytes, size_t *got) {
+  void *p = nullptr;
   {
     std::lock_guard<std::mutex> lk(h->ws_mu);
-    if (h->ws && h->ws_bytes >= bytes) {
-      void *p = h->ws;
-      *got = h->ws_bytes;
-      h->ws = nullptr;
-      h->ws_bytes = 0;
-      return p;
-    }
+    p = h->ws;
+    *got = h->ws_bytes;
+    h->ws = nullptr;
+    h->ws_bytes = 0;
   }
-  void *p = nullptr;
+  if (p && *got >= bytes) return p;
+  cudaFree(p);
   *got = bytes;
-  return cudaMalloc(&p, bytes) == cudaSuccess ? p : nullptr;
+  if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
+  cudaGetLastError();  // told by the result
+  return nullptr;
 }
 void mlp_put_workspace(qpsdm_mlp *h, void *p, size_t bytes) {
   if (!p) return;
