@@ -19,7 +19,9 @@ static std::mutex g_plan_mu;
 static std::map<std::pair<int, int>, FftPlan> g_plans;
 
 // Stockham radices of m: powers of two as 4s (and one 2), nines as 3s, then
-// 5, 7, 11, 13; a 4 and the 2 after it, and two 3s, make one group.
+// 5, 7, 11, 13; a 4 and the 2 after it, and two 3s, make one group.  A length past
+// kFftMaxHalf, which may have more groups than a plan holds, gets none: its
+// callers refuse it.
 static bool factor_radices(int m, FftPlan &p) {
   int rad[32], n = 0, r = m;
   while (r % 4 == 0) { rad[n++] = 4; r /= 4; }
@@ -29,6 +31,7 @@ static bool factor_radices(int m, FftPlan &p) {
     while (r % q == 0) { rad[n++] = q; r /= q; }
   if (r != 1) return false;
   p.nstock = 0;
+  if (m > kFftMaxHalf) return true;
   for (int i = 0; i < n; ++i) {
     const bool two = i + 1 < n && ((rad[i] == 4 && rad[i + 1] == 2) ||
                                    (rad[i] == 3 && rad[i + 1] == 3));
@@ -64,6 +67,7 @@ static bool fft_factor(int m, FftPlan &p) {
   p.n = 2 * m;
   p.m = m;
   if (!factor_radices(m, p)) return false;
+  if (m > kFftMaxHalf) return true;
   int r = m, np = 0;
   auto take = [&](int q, int prime) {
     if (r % q == 0 && r / q % prime != 0) {
@@ -344,7 +348,7 @@ extern "C" int qpsdm_fft_r2c_noalloc(const float *d_in, int n, int batch,
   if (n < 2 || (n & 1)) return QPSDM_EINVAL;
   if (batch == 0) return QPSDM_OK;
   FftPlan p{};
-  if (!fft_factor(n / 2, p)) return QPSDM_EINVAL;
+  if (!fft_factor(n / 2, p) || p.m > kFftMaxHalf) return QPSDM_EINVAL;
   float2 *tw = nullptr;
   int rc = noalloc_twiddle_ptr(&tw);
   if (rc) return rc;
