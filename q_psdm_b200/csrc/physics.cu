@@ -2521,9 +2521,11 @@ static int launch_variant(int vi, PhysicsState *s, const PhysImageArgs &a, const
 }
 
 // Tuning results shared by the engines of a process:
-// (device, nzi, nxb, dtype, nbins) -> variant.
+// (device, nzi, nxb, dtype, nbins, paired tables, batch class) -> variant.  The
+// last two decide which kernels run and in how many parts a tile's members are:
+// what is fastest for a small batch, or for float tables, is not for the others.
 static std::mutex g_tune_mu;
-static std::map<std::tuple<int, int, int, int, int>, int> g_tune;
+static std::map<std::tuple<int, int, int, int, int, int, int>, int> g_tune;
 
 // Picks the variant for this image shape: an explicit tile from the static
 // parameters, a cached result, or a timing of every variant on this batch
@@ -2540,7 +2542,10 @@ static int choose_variant(PhysicsState *s, const PhysImageArgs &a, const Physics
   }
   int dev = 0;
   cudaGetDevice(&dev);
-  const auto key = std::make_tuple(dev, a.nzi, a.nxb, s->dtype, s->nbins);
+  int parts = 0;  // log2 of the parts of 16 x 16 tiles: six classes
+  for (int n = member_split(s, a, (a.nzi + 15) / 16 * ((a.nxb + 15) / 16), b.ntr); n > 1; n /= 2)
+    ++parts;
+  const auto key = std::make_tuple(dev, a.nzi, a.nxb, s->dtype, s->nbins, (int)v.tab->paired, parts);
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);
