@@ -180,7 +180,7 @@ static void filter_table(const qpsdm_static_params &p, int nbins, float dtstar,
   const double c1 = G * (1.0 - lnG - 2.5 * lnG * lnG), c2 = G * (1.0 + 5.0 * lnG);
   const double c3 = -2.5 * G, c4 = 1.1 * G;
   out.assign((size_t)nbins * nk, make_float2(0.f, 0.f));
-  *kmax = std::max(1, std::min(nk, n4));
+  *kmax = std::max(1, std::min(nk, std::max(n3, n4)));  // (f3 > f4: a sharp edge at f3)
   for (int b = 0; b < nbins; ++b) {
     const double ts = b * (double)dtstar;
     for (int k = 1; k < nk; ++k) {
