@@ -257,12 +257,21 @@ extern "C" int qpsdm_engine_destroy(qpsdm_engine *e) {
   return QPSDM_OK;
 }
 
-extern "C" int qpsdm_set_lines(qpsdm_engine *e, const qpsdm_line_params *l, int nlines) {
-  if (!e || !l || nlines <= 0) return QPSDM_EINVAL;
-  for (int il = 0; il < nlines; ++il)
-    if (!l[il].dipx1 || !l[il].dipx2 || !l[il].dipy1 || !l[il].dipy2)
-      return fail(e, QPSDM_EINVAL, "dip fields are required");
-  DeviceGuard g(e->device);
+namespace {
+
+// A call that failed for memory or on the device half way through may have
+// freed buffers that the lines or the offset group before it used: nothing is
+// submitted, replayed or read until they have been set again.
+int unset(qpsdm_engine *e, int rc, bool lines) {
+  if (rc == QPSDM_OK || rc == QPSDM_EINVAL || rc == QPSDM_ESTATE) return rc;
+  cudaGetLastError();
+  clear_graphs(e);
+  if (lines) e->line_set = false;
+  e->offset_set = false;
+  return rc;
+}
+
+int set_lines(qpsdm_engine *e, const qpsdm_line_params *l, int nlines) {
   CK(cudaStreamSynchronize(e->s_comp));
   e->nxz = (size_t)e->p.nxi * e->p.nzi;
   if (nlines > e->lines_cap) {  // per-line dip fields and gate results
@@ -295,17 +304,24 @@ extern "C" int qpsdm_set_lines(qpsdm_engine *e, const qpsdm_line_params *l, int 
   return QPSDM_OK;
 }
 
+}  // namespace
+
+extern "C" int qpsdm_set_lines(qpsdm_engine *e, const qpsdm_line_params *l, int nlines) {
+  if (!e || !l || nlines <= 0) return QPSDM_EINVAL;
+  for (int il = 0; il < nlines; ++il)
+    if (!l[il].dipx1 || !l[il].dipx2 || !l[il].dipy1 || !l[il].dipy2)
+      return fail(e, QPSDM_EINVAL, "dip fields are required");
+  DeviceGuard g(e->device);
+  return unset(e, set_lines(e, l, nlines), true);
+}
+
 extern "C" int qpsdm_set_line(qpsdm_engine *e, const qpsdm_line_params *l) {
   return qpsdm_set_lines(e, l, 1);
 }
 
-extern "C" int qpsdm_begin_offset(qpsdm_engine *e, const qpsdm_offset_params *o) {
-  if (!e || !o) return QPSDM_EINVAL;
-  if (!e->line_set) return fail(e, QPSDM_ESTATE, "begin_offset before set_line");
-  if (o->ixstart < 0 || o->ixend > e->p.nxi || o->ixend <= o->ixstart || o->nsb <= 0 ||
-      o->nww <= 0 || o->nf1 < 0 || o->nf1 + o->nww > o->nsb / 2 + 1)
-    return fail(e, QPSDM_EINVAL, "bad offset parameters");
-  DeviceGuard g(e->device);
+namespace {
+
+int begin_offset(qpsdm_engine *e, const qpsdm_offset_params *o) {
   CK(cudaStreamSynchronize(e->s_comp));
   // -i*w frequencies accumulated in float as psdm_kernel does (w += dw).
   std::vector<float> om(o->nww);
@@ -336,6 +352,18 @@ extern "C" int qpsdm_begin_offset(qpsdm_engine *e, const qpsdm_offset_params *o)
   clear_graphs(e);
   e->offset_set = true;
   return QPSDM_OK;
+}
+
+}  // namespace
+
+extern "C" int qpsdm_begin_offset(qpsdm_engine *e, const qpsdm_offset_params *o) {
+  if (!e || !o) return QPSDM_EINVAL;
+  if (!e->line_set) return fail(e, QPSDM_ESTATE, "begin_offset before set_line");
+  if (o->ixstart < 0 || o->ixend > e->p.nxi || o->ixend <= o->ixstart || o->nsb <= 0 ||
+      o->nww <= 0 || o->nf1 < 0 || o->nf1 + o->nww > o->nsb / 2 + 1)
+    return fail(e, QPSDM_EINVAL, "bad offset parameters");
+  DeviceGuard g(e->device);
+  return unset(e, begin_offset(e, o), false);
 }
 
 namespace {
