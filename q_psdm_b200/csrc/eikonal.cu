@@ -203,10 +203,18 @@ __device__ __forceinline__ float eik_update(float a, float b, float c, float f) 
 // sources: 256 sweeps over every node, in global memory, took 70 ms; over listed
 // blocks, one update a visit, 15.4 ms in 224 sweeps; now 5.4 ms in 80.  With 1,
 // 2, 4, 8, 16 updates a visit at most, and 7 ms of t* in each: 26.5, 20.8, 14.9,
-// 13.1, 12.9 ms.  Eight: the FP32 update's rounding lets values creep below the
-// fixed point, and the fewer updates, the less they do (error 0.6 to 1.3 of the
-// full sweeps', 0.98 on average); with 16 they end up to 4 times as far from the
-// full sweeps' values as two runs of those from each other, with 8 at most 3 times.
+// 13.1, 12.9 ms.
+//
+// The price is in T's rounding.  The FP32 update rounds by some eps T^2 / f, a
+// node keeps the lowest of its values, and the order of updates decides how far
+// below the fixed point it creeps: T's error against 64 bits, relative 2e-5 to
+// 5e-4, is 1.2 times the full sweeps' (geometric mean of 64 models, 3 to 8 sources
+// each; 0.9 to 1.6 in most, 2.7 where the full sweeps' was 1.6e-5), t*'s 1.03 to
+// 1.09 times.  One update a visit from global memory had 1.03 times (1.26 at
+// most) in 23 ms, ignoring changes below 1e-6 of T instead of 1e-7 1.0 times (2.1)
+// in this kernel's time.  Neither was taken: t* takes its upwind neighbours by T,
+// so with any other T near ties fall the other way, and results would leave this
+// solver's by some 1e-4 of t*, more than FP32 rounding accounts for.
 constexpr int kEikInner = 8;
 __global__ void __launch_bounds__(kEikThreads)
     k_eik_relax(const float *__restrict__ F, float *__restrict__ T, EikBlocks B, int sweep) {
