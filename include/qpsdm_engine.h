@@ -173,6 +173,9 @@ int qpsdm_engine_destroy(qpsdm_engine *e);
 const char *qpsdm_last_error(const qpsdm_engine *e);
 
 /* ---- line / offset state ---------------------------------------------------*/
+/* A call of this section that fails with QPSDM_ENOMEM or QPSDM_ECUDA leaves the
+ * engine without lines (set_line(s)) or offset group: submits and image reads
+ * return QPSDM_ESTATE until the call has succeeded. */
 
 /* Replaces get_ttt_all x2 + the dip/nf3/Q uploads of qpsdm()
  * (src/q-psdm.cu:1449-1515). */
